@@ -25,24 +25,31 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_ref", "libddecal_ref.so")
-REFERENCE = os.environ.get("DP3_REFERENCE", "/root/reference")
+# The reference tree, or "" where its solver sources are not there (a mount
+# point without the tree is no reference).
+_TREE = os.environ.get("DP3_REFERENCE", "/root/reference")
+REFERENCE = _TREE if os.path.isdir(os.path.join(_TREE, "ddecal", "gain_solvers")) else ""
 
 DIAGONAL_DUO, DIAGONAL_FULL, SCALAR_UNI, SCALAR_DUO, SCALAR_FULL, FULL_JONES = range(6)
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference library is not built and its sources are not here."""
+
+
 def available():
-    return os.path.exists(LIB_PATH) or os.path.isdir(REFERENCE)
+    return os.path.exists(LIB_PATH) or bool(REFERENCE)
 
 
 def build(force=False):
     """Compiles _ref/libddecal_ref.so from the reference tree when present."""
-    if os.path.isdir(REFERENCE):
+    if REFERENCE:
         cmd = ["make", "-C", HERE, f"REF={REFERENCE}", "_ref/libddecal_ref.so"]
         if force:
             cmd.insert(1, "-B")
         subprocess.check_call(cmd, stdout=subprocess.DEVNULL)
     if not os.path.exists(LIB_PATH):
-        raise RuntimeError(f"{LIB_PATH} is missing and the reference tree is absent")
+        raise ReferenceMissing(f"{LIB_PATH} is missing and the reference tree is absent")
     return LIB_PATH
 
 
