@@ -92,17 +92,13 @@ __host__ __device__ __forceinline__ uint64_t SlabElem(uint32_t R, uint32_t W, ui
 
 // pipe_kernel work item: rows [row_lo, row_hi) of the (t, channel) rows of
 // the tile of runs [r0, r0 + n_runs) of a slab; fragments of one CTA that
-// share a slab form a visit (one partial slot).
+// share a slab form a visit (one partial slot). meta: the tile's antennas
+// (TileMeta), first word / 4 and bytes.
 struct Frag {
-  uint32_t slab, r0, n_runs, flags, row_lo, row_hi, visit, tile;
-  uint32_t group_end[2];  // direct reduction: end run (exclusive) of groups
-                          // 0..7, one byte each; groups partition [0, n_runs)
+  uint32_t slab, r0, n_runs, flags, row_lo, row_hi, visit, tile, meta, meta_bytes, pad[2];
 };
-constexpr uint32_t kFragDirect = 1u;  // runs split into <= 8 groups, each with
-                                      // distinct first and second antennas
-constexpr uint32_t kMaxGroups = 8;
-constexpr uint32_t kFragPower = 2u;   // the fragment adds its tile's precomputed
-                                      // model powers sum |M|^2 (one per tile)
+constexpr uint32_t kFragPower = 1u;  // the fragment adds its tile's precomputed
+                                     // model powers sum |M|^2 (one per tile)
 
 struct Visit {
   uint32_t slab, run_lo, run_hi, pad;
@@ -1081,6 +1077,12 @@ struct NeumaierSum {  // compensated FP32 summation (two-sum)
       c += (x - t) + s;
     s = t;
   }
+  // Adds the sum of the lane `o` away (which adds this one).
+  __device__ __forceinline__ void Join(uint32_t lanes, int o) {
+    const float xs = __shfl_xor_sync(lanes, s, o), xc = __shfl_xor_sync(lanes, c, o);
+    Add(xs);
+    c += xc;
+  }
   __device__ __forceinline__ float Value() const { return s + c; }
 };
 
@@ -1331,12 +1333,41 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(const FinParams p) {
 // error flag that the host reports as DDSOLVE_E_TIMEOUT, and all later waits
 // of that CTA return at once so that the kernel still ends.
 // ---------------------------------------------------------------------------
-constexpr int kPipeConsumerWarps = 7;
-constexpr int kPipeRuns = kPipeConsumerWarps * 32;  // runs per tile
-constexpr int kPipeThreads = kPipeRuns + 32;         // + one producer warp
+// Consumer warps of a CTA, beside one producer warp: kWarps (168 registers a
+// thread), or kWideWarps (255) for more than kPipeDirs2 * 4 directions.
+constexpr int kWarps = 11, kWideWarps = 7;
+// Directions per lane at most (2 and 4 correlations): gains, sums and the
+// model row of that many fit a thread's 168 registers; with kWideWarps, gains
+// and sums fit 255.
+constexpr uint32_t kPipeDirs2 = 5, kPipeDirs4 = 3, kPipeDirsWide = 12;
 constexpr int kPipeMaxStages = 8;
-static_assert(kPipeRuns <= 256 && kPipeRuns % 32 == 0, "tree reductions assume <= 256 consumers");
 constexpr uint64_t kWaitBudgetNs = 4000000000ull;
+
+// Device counters of pipe_kernel, each polled word on a cache line of its
+// own. The error flag (a bounded wait ran out). Arrivals of CTAs whose partial
+// slots are written, and (64 bits) of CTAs that have finalised the pass, with
+// the arrivals that saw non-finite solutions in the high half: both count on
+// through the passes and launches, a multiple of the grid between launches.
+// The number of passes whose control step is done and, beside it, its verdict.
+constexpr uint32_t kCntError = 1, kCntArrive = 32, kCntEpoch = 64, kCntVerdict = 65,
+                   kCntFinal = 96;
+constexpr uint32_t kCounterWords = 128;
+constexpr size_t kCounterBytes = kCounterWords * 4;
+constexpr uint32_t kVerdictStop = 1u;  // the solve ends with this pass
+constexpr uint32_t kVerdictNear = 2u;  // it may end with the next one
+// Passes per launch at most: the launch ends within a bounded time, and other
+// contexts' kernels get the GPU.
+constexpr uint32_t kItersPerLaunch = 64;
+
+// The partial slots of one (channel block, sub-solution) in the finalisation:
+// a range of visits, or a list in fin_visits; its direction; and its gain-table
+// entry (table * 256 + direction) when it has just one, else kManyEntries.
+struct FinList {
+  uint32_t first;  // first visit, or first index in fin_visits
+  uint32_t count;  // | kFinRange
+  uint32_t dir, entry;
+};
+constexpr uint32_t kFinRange = 0x80000000u, kManyEntries = 0xFFFFFFFFu;
 
 struct PipeParams {
   const SlabDesc* slabs;
@@ -1354,25 +1385,28 @@ struct PipeParams {
   uint32_t gain_stride;   // float2 per antenna in a gain table (PipeGainStride)
   uint32_t stages;
   uint32_t acc_floats;    // n_ant * acc_stride = one partial slot
-  uint32_t owner_groups;  // direction groups per antenna in the sorted reduction
+  const uint32_t* metas;  // TileMeta blocks
+  uint32_t meta_words;    // words of a TileMeta buffer in shared memory
   uint32_t n_gbuf;        // gain table buffers in shared memory (1 or 2)
-  const float* powers;    // model powers per tile [tile][dir][corr][kPipeRuns],
+  const float* powers;    // model powers per tile [tile][dir][runs of a tile][corr],
                           // or null: accumulated in the row loop
   uint32_t power_floats;  // floats per tile in `powers`
   // shared-memory layout (byte offsets)
-  uint32_t off_acc, off_gtab, off_stg, off_cnt, off_off, off_pair, off_ent,
-      off_wsum, off_stages;
-  const uint32_t* fin_off;
+  uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
+  const FinList* fin_lists;    // [n_cb * n_sub]
   const uint32_t* fin_visits;
-  const uint32_t* fin_first;  // first visit of each list when all lists are ranges, else null
-  const uint32_t* dir_of_sub;
   uint32_t* cb_flag;     // channel block holds non-finite solutions
   double* cb_avg;        // replacement value for them (MakeSolutionsFinite)
   uint32_t* cb_newflag;  // set during the finalisation that produced them
   double* block_sum;     // per-CTA norm partials
   uint32_t* block_cnt;
-  uint32_t* counters;    // [0] CTAs finalised, [1] error flag, [2] grid barrier
+  uint32_t* counters;    // kCounterWords words, see there
   double2* next_out;
+  // Passes of this launch: a solve's iterations until it stops, or (host
+  // mode) a chain of next-solutions passes, pass k + 1 starting from the
+  // output of pass k, which goes to next_out + k * out_stride.
+  uint32_t n_iters;
+  size_t out_stride;
   int32_t host_mode;
   int32_t fin_mode;      // FinFused / FinStepOnly / FinAssignOnly
   const DevSettings* settings;
@@ -1380,14 +1414,42 @@ struct PipeParams {
   double* step_magnitudes;
   cudaGraphConditionalHandle handle;
   int32_t use_handle;
-  // Independent intervals (batched solve): interval g owns channel blocks
-  // [group_cb[g], group_cb[g + 1]) (cb_group[cb] = g), its loop state
-  // state[g], step magnitudes step_magnitudes[g * mags_stride] and norm
-  // partials block_sum[g * gridDim.x + CTA]. One interval: n_groups = 1.
+  // Independent intervals (batched solve): interval g owns the channel blocks
+  // with cb_group[cb] = g, its loop state state[g] and step magnitudes
+  // step_magnitudes[g * mags_stride]. One interval: n_groups = 1, and a norm
+  // partial per CTA.
   uint32_t n_groups;
   const uint32_t* cb_group;
-  const uint32_t* group_cb;
   uint32_t mags_stride;
+  // Several intervals: their finalisation items in runs of at most 32 of one
+  // interval, a warp's round each: first item, count << 24 | interval. The
+  // norm partials are per chunk then, interval g's at [group_chunk[g],
+  // group_chunk[g + 1]).
+  uint32_t n_chunks;
+  const uint2* chunks;
+  const uint32_t* group_chunk;
+};
+
+// The head of pipe_kernel's shared memory.
+struct PipeShared {
+  uint64_t full[kPipeMaxStages], empty[kPipeMaxStages];  // ring
+  uint64_t gfull[2], gfree[2];  // gain table buffer loaded / released
+  uint64_t mfree[2];            // antenna buffer released
+  // Thread 0 polls the grid's counters for its CTA and passes the news on to
+  // the consumers: every partial slot of the pass is written; the pass is
+  // finished (with `stop`: so is the launch). One phase per pass each. The
+  // producer, which no barrier keeps within a phase of the consumers, reads
+  // the number of finished passes instead.
+  uint64_t flushed, ready;
+  double sum[16];  // the warps' norm partials
+  uint32_t cnt[32];
+  uint32_t flag[2];
+  volatile uint32_t stop, passes;
+  volatile int err;
+  // thread 0: the counters before the launch, non-finite arrivals so far, the
+  // verdict on the pass before
+  uint32_t epoch0, final0, arrive0, bad_seen, verdict;
+  PipeParams params;
 };
 
 // A fragment of an interval that has stopped: skipped by the producer and the
@@ -1400,6 +1462,19 @@ __device__ __forceinline__ bool FragFrozen(const PipeParams& p, uint32_t slab) {
 
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// A pointer to shared memory from its 32-bit address: passed so to functions
+// kept out of line, whose pointer arguments would be read as generic memory.
+template <typename T>
+__device__ __forceinline__ T* SharedPtr(uint32_t at) {
+  return static_cast<T*>(__cvta_shared_to_generic(at));
+}
+// The thread index, read anew: what is computed from it is not carried through
+// (or hoisted out of) the loops around.
+__device__ __forceinline__ int FreshTid() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
 }
 __device__ __forceinline__ void MbarInit(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)),
@@ -1435,6 +1510,19 @@ __device__ __forceinline__ void BulkCopyG2S(void* dst, const void* src,
       "l"(src), "r"(bytes), "r"(SmemAddr(bar))
       : "memory");
 }
+// Orders this thread's generic accesses to global memory (its own writes, or
+// writes it has acquired) against bulk copies of the same memory.
+__device__ __forceinline__ void FenceProxyAsync() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t LoadAcquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void StoreRelease(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 __device__ __forceinline__ uint64_t GlobalTimerNs() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1446,24 +1534,55 @@ __device__ __forceinline__ uint64_t GlobalTimerNs() {
 // the non-aligned `barrier.sync 1, 224` let six waiting warps through while
 // the seventh was still busy, and so did `bar.sync` after a loop that only
 // one warp ran; waits of that kind are done by every warp instead.
+template <int W>
 __device__ __forceinline__ void ConsumerBarrier() {
   __syncwarp();
-  asm volatile("bar.sync 1, %0;" ::"n"(kPipeRuns) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory");
 }
 
 // Bounded wait on an mbarrier phase. Returns false on timeout (or when the CTA
 // is already in error), after recording the error.
-__device__ __forceinline__ bool PipeWait(uint64_t* bar, uint32_t parity,
-                                      volatile int* s_err, uint32_t* g_err) {
+__device__ __forceinline__ bool PipeWaitSlow(uint64_t* bar, uint32_t parity, volatile int* s_err,
+                                             uint32_t* g_err) {
+  uint64_t t0 = 0;
+  for (uint32_t n = 1;; ++n) {
+    if (MbarTryWait(bar, parity)) return true;
+    if ((n & 15u) == 0) {  // (reading the timer is slow)
+      if (*s_err) return false;
+      const uint64_t t = GlobalTimerNs();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kWaitBudgetNs) {
+        *s_err = 1;
+        atomicExch(g_err, 1u);
+        return false;
+      }
+    }
+  }
+}
+__device__ __forceinline__ bool PipeWait(uint64_t* bar, uint32_t parity, volatile int* s_err,
+                                         uint32_t* g_err) {
   if (MbarTryWait(bar, parity)) return true;
+  return PipeWaitSlow(bar, parity, s_err, g_err);
+}
+
+__device__ __forceinline__ uint64_t LoadAcquire64(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// Thread 0's bounded wait until reached() holds; false when it ran out or an
+// error is flagged.
+template <typename Reached>
+__device__ __forceinline__ bool GridWait(uint32_t* counters, const Reached& reached) {
   const uint64_t t0 = GlobalTimerNs();
   for (uint32_t n = 1;; ++n) {
-    if (*s_err) return false;
-    if (MbarTryWait(bar, parity)) return true;
-    if ((n & 63u) == 0 && GlobalTimerNs() - t0 > kWaitBudgetNs) {
-      *s_err = 1;
-      atomicExch(g_err, 1u);
-      return false;
+    if (reached()) return true;
+    if ((n & 63u) == 0) {
+      if (static_cast<volatile uint32_t*>(counters)[kCntError]) return false;
+      if (GlobalTimerNs() - t0 > kWaitBudgetNs) {
+        atomicExch(&counters[kCntError], 1u);
+        return false;
+      }
     }
   }
 }
@@ -1490,31 +1609,31 @@ __device__ __forceinline__ void LoadVisShared(const char* base, uint32_t idx,
 // denominators (NPOL real values each), so that one direction's update is
 // one vector read-modify-write of each (stride = 4 mod 8: distinct
 // shared-memory banks for consecutive antennas).
-template <int NPOL>
-__device__ __forceinline__ void AccAdd(float* acc, uint32_t a, uint32_t stride, uint32_t n_dir,
-                                       uint32_t d, const float2 (&num)[NPOL],
-                                       const float (&den)[NPOL]) {
-  float* row = acc + size_t(a) * stride;
+template <int NPOL, bool HAS_DEN>
+__device__ __forceinline__ void AccAdd(float* row, uint32_t n_dir, uint32_t d,
+                                       const float2 (&num)[NPOL], const float (&den)[NPOL]) {
   if constexpr (NPOL == 2) {
     float4* pn = reinterpret_cast<float4*>(row) + d;
+    float2* pd = reinterpret_cast<float2*>(row + 4 * n_dir) + d;
     float4 v = *pn;
+    float2 w = HAS_DEN ? *pd : make_float2(0.f, 0.f);
     v.x += num[0].x;
     v.y += num[0].y;
     v.z += num[1].x;
     v.w += num[1].y;
     *pn = v;
-    float2* pd = reinterpret_cast<float2*>(row + 4 * n_dir) + d;
-    float2 w = *pd;
-    w.x += den[0];
-    w.y += den[1];
-    *pd = w;
+    if constexpr (HAS_DEN) {
+      w.x += den[0];
+      w.y += den[1];
+      *pd = w;
+    }
   } else {
     float2* pn = reinterpret_cast<float2*>(row) + d;
     float2 v = *pn;
     v.x += num[0].x;
     v.y += num[0].y;
     *pn = v;
-    row[2 * n_dir + d] += den[0];
+    if constexpr (HAS_DEN) row[2 * n_dir + d] += den[0];
   }
 }
 __host__ __device__ constexpr uint32_t AccNumOffset(uint32_t npol, uint32_t d, uint32_t q) {
@@ -1542,47 +1661,292 @@ __device__ __forceinline__ void LoadGains(const float2* gtab, uint32_t ant, uint
 // Writes the FP32 gain-table entries of solution (cb, ant, s): one entry per
 // gain table of that channel block whose slab uses sub-solution s.
 template <int NPOL>
-__device__ __forceinline__ void WriteTables(const PipeParams& p, uint32_t cb,
-                                            uint32_t ant, uint32_t s,
+__device__ __forceinline__ void WriteTables(const PipeParams& p, uint32_t cb, uint32_t ant,
+                                            uint32_t s, uint32_t entry,
                                             const double2 (&v)[NPOL]) {
-  const uint32_t k0 = p.tab_off[cb * p.n_sub + s];
-  const uint32_t k1 = p.tab_off[cb * p.n_sub + s + 1];
-  for (uint32_t k = k0; k < k1; ++k) {
-    const uint32_t e = p.tab_ent[k];
+  auto put = [&](uint32_t e) {
     float2* t = p.tables + size_t(e >> 8) * p.table_f2 + size_t(ant) * p.gain_stride +
                 (e & 255u) * NPOL;
 #pragma unroll
     for (int q = 0; q < NPOL; ++q) t[q] = make_float2(float(v[q].x), float(v[q].y));
+  };
+  if (entry != kManyEntries) {
+    put(entry);
+    return;
+  }
+  const uint32_t k1 = p.tab_off[cb * p.n_sub + s + 1];
+  for (uint32_t k = p.tab_off[cb * p.n_sub + s]; k < k1; ++k) put(p.tab_ent[k]);
+}
+
+// |diff / old| of the AssignSolutions norm; false where the quotient by the
+// inverse of `old` would not be finite. Within the range where neither square
+// can over- or underflow it is one division and one square root.
+__device__ __noinline__ bool StepNormSlow(double2 old, double2 diff, double& r) {
+  const double2 inv = dinv(old);
+  if (!dfinite(inv)) return false;
+  const double2 q = dmul(diff, inv);
+  r = hypot(q.x, q.y);
+  return true;
+}
+__device__ __forceinline__ bool StepNorm(double2 old, double2 diff, double& r) {
+  const double o2 = old.x * old.x + old.y * old.y, d2 = diff.x * diff.x + diff.y * diff.y;
+  if (o2 > 1e-200 && o2 < 1e200 && d2 < 1e200 && (d2 > 1e-200 || d2 == 0.0)) {
+    r = sqrt(d2 / o2);
+    return true;
+  }
+  return StepNormSlow(old, diff, r);
+}
+
+// One item's sums in a partial slot: NPOL complex numerators and NPOL real
+// denominators (AccAdd), as one vector load of each.
+template <int NPOL>
+__device__ __forceinline__ void LoadSlot(const float* num, const float* den,
+                                         float (&v)[NPOL * 3]) {
+  if constexpr (NPOL == 2) {
+    const float4 n = __ldcg(reinterpret_cast<const float4*>(num));
+    const float2 d = __ldcg(reinterpret_cast<const float2*>(den));
+    v[0] = n.x;
+    v[1] = n.y;
+    v[2] = n.z;
+    v[3] = n.w;
+    v[4] = d.x;
+    v[5] = d.y;
+  } else {
+    const float2 n = __ldcg(reinterpret_cast<const float2*>(num));
+    v[0] = n.x;
+    v[1] = n.y;
+    v[2] = __ldcg(den);
   }
 }
 
-// Grid-wide finalisation of pipe_kernel, after the grid barrier: the
-// consumer threads of all CTAs take (channel block, antenna, sub-solution)
-// items in a grid-stride loop, one round per independent interval (one round
-// for a single interval): fixed-order compensated merge of the item's
-// partial slots, FP64 add-back and division (IterativeDiagonalSolver.cc:206-221,
-// IterativeScalarSolver.cc:184-194), SolverBase::Step (SolverBase.cc:88-158),
-// the AssignSolutions norm (SolverBase.cc:234-285), and the FP32 gain tables
-// of the next iteration. The last CTA to finish sums each interval's per-CTA
-// norms in CTA order, runs ReachedStoppingCriterion / DetectStall (SolverBase.h:274-285,
-// SolverBase.cc:63-86), and prepares the next iteration's
-// MakeSolutionsFinite{1,2}Pol (SolverBase.cc:316-371) for channel blocks that
-// got non-finite solutions. With device constraints the work is split by
-// p.fin_mode: kFinStepOnly (pipe_kernel) stops after the step, writing the
-// stepped solutions to next_out; kFinAssignOnly (assign_kernel) starts from
-// the constrained ones in next_out.
-template <int NPOL>
-__device__ __forceinline__ void FinalizeDistributed(const PipeParams& p, int ctid,
-                                                 double* s_sum, uint32_t* s_cnt,
-                                                 uint32_t* s_last) {
+// Sums (and the or of `flag`) over the consumer threads of a CTA in a fixed
+// order; valid in thread 0. s_cnt: two words per warp.
+template <int W>
+__device__ __forceinline__ void BlockNorm(int ctid, double& sum, uint32_t& cnt, bool& flag,
+                                          double* s_sum, uint32_t* s_cnt) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
+  }
+  flag = __any_sync(0xFFFFFFFFu, flag);
+  if ((ctid & 31) == 0) {
+    s_sum[ctid >> 5] = sum;
+    s_cnt[2 * (ctid >> 5)] = cnt;
+    s_cnt[2 * (ctid >> 5) + 1] = flag ? 1u : 0u;
+  }
+  ConsumerBarrier<W>();
+  if (ctid == 0)
+    for (int w = 1; w < W; ++w) {
+      sum += s_sum[w];
+      cnt += s_cnt[2 * w];
+      flag = flag || s_cnt[2 * w + 1] != 0;
+    }
+}
+
+// An interval's loop state, read and written past L1: within one launch the
+// CTA that finishes a pass changes from pass to pass.
+__device__ __forceinline__ LoopState LoadState(const LoopState* s) {
+  static_assert(sizeof(LoopState) % 8 == 0, "copied in 8-byte words");
+  LoopState r;
+  const uint2* src = reinterpret_cast<const uint2*>(s);
+  uint2* dst = reinterpret_cast<uint2*>(&r);
+#pragma unroll
+  for (size_t i = 0; i < sizeof(LoopState) / 8; ++i) dst[i] = __ldcg(src + i);
+  return r;
+}
+__device__ __forceinline__ void StoreState(LoopState* s, const LoopState& v) {
+  uint2* dst = reinterpret_cast<uint2*>(s);
+  const uint2* src = reinterpret_cast<const uint2*>(&v);
+#pragma unroll
+  for (size_t i = 0; i < sizeof(LoopState) / 8; ++i) __stcg(dst + i, src[i]);
+}
+
+// The control step of a pass, run by one CTA after all have finalised it:
+// sums each interval's per-CTA norms in a fixed order, runs
+// ReachedStoppingCriterion / DetectStall (SolverBase.h:274-285,
+// SolverBase.cc:63-86), and (`bad`) prepares the next iteration's
+// MakeSolutionsFinite{1,2}Pol (SolverBase.cc:316-371) of the channel blocks
+// that got non-finite solutions. Returns the verdict (in thread 0). All
+// consumer threads of the CTA take part; s_flag: two words.
+template <int W, int NPOL>
+__device__ __forceinline__ uint32_t ControlPass(const PipeParams& p, int ctid, bool bad,
+                                                double* s_sum, uint32_t* s_cnt,
+                                                uint32_t* s_flag) {
+  const DevSettings st = *p.settings;
+  const bool error = static_cast<volatile uint32_t*>(p.counters)[kCntError] != 0;
+  if (bad) {
+    // Replacement values for channel blocks with new non-finite solutions:
+    // mean |pol 0| over finite pairs; the gain tables take the replacement
+    // now, the solutions when the next finalisation reads them.
+    const uint32_t n_items_cb = p.n_ant * p.n_sub;
+    for (uint32_t cb = 0; cb < p.n_cb; ++cb) {
+      if (static_cast<volatile uint32_t*>(p.cb_newflag)[cb] == 0) continue;
+      double asum = 0.0;
+      uint32_t acnt = 0;
+      for (uint32_t i = ctid; i < n_items_cb; i += (W * 32)) {
+        const double2* sol = p.solutions + (size_t(cb) * n_items_cb + i) * NPOL;
+        bool ok = true;
+        double2 v[NPOL];
+#pragma unroll
+        for (int q = 0; q < NPOL; ++q) {
+          v[q] = __ldcg(sol + q);
+          ok = ok && dfinite(v[q]);
+        }
+        if (ok) {
+          asum += hypot(v[0].x, v[0].y);
+          ++acnt;
+        }
+      }
+      bool unused = false;
+      BlockNorm<W>(ctid, asum, acnt, unused, s_sum, s_cnt);
+      if (ctid == 0) s_sum[0] = acnt == 0 ? 1.0 : asum / double(acnt);
+      ConsumerBarrier<W>();
+      const double avg = s_sum[0];
+      for (uint32_t i = ctid; i < n_items_cb; i += (W * 32)) {
+        const double2* sol = p.solutions + (size_t(cb) * n_items_cb + i) * NPOL;
+        bool ok = true;
+#pragma unroll
+        for (int q = 0; q < NPOL; ++q) ok = ok && dfinite(__ldcg(sol + q));
+        if (!ok) {
+          double2 r[NPOL];
+#pragma unroll
+          for (int q = 0; q < NPOL; ++q) r[q] = make_double2(avg, 0.0);
+          WriteTables<NPOL>(p, cb, i / p.n_sub, i % p.n_sub, kManyEntries, r);
+        }
+      }
+      ConsumerBarrier<W>();
+      if (ctid == 0) {
+        __stcg(p.cb_avg + cb, avg);
+        __stcg(p.cb_flag + cb, 1u);
+        p.cb_newflag[cb] = 0u;
+      }
+      ConsumerBarrier<W>();
+    }
+    FenceProxyAsync();
+    ConsumerBarrier<W>();
+  }
+  uint32_t verdict = 0;
+  if (p.n_groups == 1) {
+    if (ctid >= 32) return 0u;
+    LoopState ls = LoadState(p.state);  // (issued with the norms' loads)
+    double sum = 0.0;
+    uint32_t cnt = 0;
+    constexpr int kLoads = 5;  // 160 CTAs per round
+    for (uint32_t b0 = ctid; b0 < gridDim.x; b0 += 32 * kLoads) {
+      double v[kLoads];
+      uint32_t c[kLoads];
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) {
+        const uint32_t b = min(b0 + 32 * k, gridDim.x - 1);
+        v[k] = __ldcg(p.block_sum + b);
+        c[k] = __ldcg(p.block_cnt + b);
+      }
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k)
+        if (b0 + 32 * k < gridDim.x) {
+          sum += v[k];
+          cnt += c[k];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+      cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
+    }
+    if (ctid == 0) {
+      bool stop = ControlStep(ls, st, sum, cnt, p.step_magnitudes);
+      if (error) {
+        ls.done = 1;
+        stop = true;
+      }
+      StoreState(p.state, ls);
+      // within a factor of two of a criterion (or not comparable with it)
+      const double mag = cnt == 0 ? 0.0 : sum / st.step_size / double(cnt);
+      const bool near_end = !(mag > 2.0 * st.accuracy) ||
+                            (st.detect_stalling &&
+                             !(ls.step_mean > 2.0 * st.step_diff_sigma *
+                                                  sqrt(ls.step_var / double(ls.n_var_count))));
+      verdict = (stop ? kVerdictStop : 0u) | (near_end ? kVerdictNear : 0u);
+    }
+    return verdict;
+  }
+  // Several intervals: one warp per interval still going sums its norm
+  // partials (in chunk order per lane) and runs its control step; the loop
+  // goes on while any interval does.
+  ConsumerBarrier<W>();
+  if (ctid == 0) s_flag[0] = 0u;
+  ConsumerBarrier<W>();
+  const int lane = ctid & 31;
+  for (uint32_t g = uint32_t(ctid >> 5); g < p.n_groups; g += W) {
+    LoopState ls = LoadState(p.state + g);
+    if (ls.done) continue;
+    double sum = 0.0;
+    uint32_t cnt = 0;
+    const uint32_t c1 = p.group_chunk[g + 1];
+#pragma unroll 4
+    for (uint32_t c = p.group_chunk[g] + lane; c < c1; c += 32) {
+      sum += __ldcg(p.block_sum + c);
+      cnt += __ldcg(p.block_cnt + c);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+      cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
+    }
+    if (lane == 0) {
+      bool stop = ControlStep(ls, st, sum, cnt, p.step_magnitudes + size_t(g) * p.mags_stride);
+      if (error) {
+        ls.done = 1;
+        stop = true;
+      }
+      StoreState(p.state + g, ls);
+      __threadfence();
+      if (!stop) atomicOr(&s_flag[0], 1u);
+    }
+    __syncwarp();
+  }
+  ConsumerBarrier<W>();
+  return s_flag[0] ? kVerdictNear : kVerdictStop | kVerdictNear;
+}
+
+// Grid-wide finalisation of a pass of pipe_kernel, after the grid barrier:
+// the consumer threads of all CTAs take (channel block, antenna,
+// sub-solution) items, warp by warp over the CTAs, one round per independent
+// interval (one round for a single interval): fixed-order compensated merge
+// of the item's partial slots, FP64 add-back and division
+// (IterativeDiagonalSolver.cc:206-221, IterativeScalarSolver.cc:184-194),
+// SolverBase::Step (SolverBase.cc:88-158), the AssignSolutions norm
+// (SolverBase.cc:234-285), and the FP32 gain tables of the next iteration.
+// With device constraints the work is split by p.fin_mode: kFinStepOnly
+// (pipe_kernel) stops after the step, writing the stepped solutions to
+// next_out; kFinAssignOnly (assign_kernel) starts from the constrained ones
+// in next_out. `it` is the pass of the launch. Solutions change between the
+// passes of a launch, so they are read past L1. wait_slots() is the grid
+// barrier, false when the launch ends there; what an item needs besides its
+// slots is read before it. Returns false with it, else sets `bad` (in thread
+// 0) when the CTA's items got non-finite solutions.
+// Bound by latency (7440 items of a 62-station, 12-block, 10-direction
+// interval are one item per thread of a quarter of the grid; a dependent read
+// of L2 costs 0.7 us): the items are spread over all CTAs and an item's slots
+// are loaded together, numerators and denominators as one vector each.
+template <int W, int NPOL, typename WaitSlots>
+__device__ __forceinline__ bool FinalizeDistributed(const PipeParams& p, uint32_t it, int ctid,
+                                                    double* s_sum, uint32_t* s_cnt, bool& bad,
+                                                    const WaitSlots& wait_slots) {
   const DevSettings st = *p.settings;
   const uint32_t n_items_cb = p.n_ant * p.n_sub;
   const uint32_t n_items = p.n_cb * n_items_cb;
+  const bool chained = p.host_mode && it > 0;
+  const double2* sol_in =
+      chained ? p.next_out + size_t(it - 1) * p.out_stride : p.solutions;
+  double2* nxt_out = p.next_out + size_t(p.host_mode ? it : 0u) * p.out_stride;
   double nsum = 0.0;
   uint32_t ncnt = 0;
+  bad = false;
   // One item: the merged sums and the old solutions in, the next solutions,
   // their norm terms, the gain tables and the non-finite flag out.
-  auto finish = [&](uint32_t item, uint32_t cb, uint32_t ant, uint32_t s,
+  auto finish = [&](uint32_t item, uint32_t cb, uint32_t ant, uint32_t s, uint32_t entry,
                     const double2 (&old_in)[NPOL], const NeumaierSum (&nr)[NPOL],
                     const NeumaierSum (&ni)[NPOL], const NeumaierSum (&dn)[NPOL]) {
     double2* sol = p.solutions + size_t(item) * NPOL;
@@ -1595,8 +1959,8 @@ __device__ __forceinline__ void FinalizeDistributed(const PipeParams& p, int cti
     }
     // the lazy MakeSolutionsFinite of a solve (next-solutions passes use the
     // solutions they are given, as PerformIteration does)
-    if (!pair_ok && !p.host_mode && p.cb_flag[cb]) {
-      const double rv = p.cb_avg[cb];
+    if (!pair_ok && !p.host_mode && __ldcg(p.cb_flag + cb)) {
+      const double rv = __ldcg(p.cb_avg + cb);
 #pragma unroll
       for (int q = 0; q < NPOL; ++q) old[q] = make_double2(rv, 0.0);
     }
@@ -1611,13 +1975,13 @@ __device__ __forceinline__ void FinalizeDistributed(const PipeParams& p, int cti
             double(float(old[q].y)) + double(ni[q].Value()) / double(den));
       }
     }
-    double2* out = p.next_out + size_t(item) * NPOL;
+    double2* out = nxt_out + size_t(item) * NPOL;
     if (p.host_mode) {
 #pragma unroll
       for (int q = 0; q < NPOL; ++q) out[q] = nxt[q];
       // the gain tables of a chained next pass, which starts from `nxt`
       // (every other launch rebuilds them from its own solutions first)
-      WriteTables<NPOL>(p, cb, ant, s, nxt);
+      WriteTables<NPOL>(p, cb, ant, s, entry, nxt);
       return;
     }
     if (p.fin_mode == kFinAssignOnly) {
@@ -1648,30 +2012,18 @@ __device__ __forceinline__ void FinalizeDistributed(const PipeParams& p, int cti
         return;
       }
     }
-    if (NPOL == 1) {
-      if (old[0].x != 0.0 || old[0].y != 0.0) {
-        const double2 diff = dmul(
-            make_double2(nxt[0].x - old[0].x, nxt[0].y - old[0].y), dinv(old[0]));
-        const double a = hypot(diff.x, diff.y);
-        if (isfinite(a)) {
-          nsum += a;
-          ncnt += 1;
-        }
+    {  // (a polarization pair counts when both do; a zero solution does not)
+      double r = 0.0;
+      bool ok = true;
+#pragma unroll
+      for (int q = 0; q < NPOL; ++q) {
+        double rq = 0.0;
+        ok = StepNorm(old[q], make_double2(nxt[q].x - old[q].x, nxt[q].y - old[q].y), rq) && ok;
+        r += rq;
       }
-    } else {
-      const double2 inv0 = dinv(old[0]);
-      const double2 inv1 = dinv(old[NPOL - 1]);
-      if (dfinite(inv0) && dfinite(inv1)) {
-        const double2 d0 =
-            dmul(make_double2(nxt[0].x - old[0].x, nxt[0].y - old[0].y), inv0);
-        const double2 d1 = dmul(make_double2(nxt[NPOL - 1].x - old[NPOL - 1].x,
-                                             nxt[NPOL - 1].y - old[NPOL - 1].y),
-                                inv1);
-        const double sumabs = hypot(d0.x, d0.y) + hypot(d1.x, d1.y);
-        if (isfinite(sumabs)) {
-          nsum += sumabs;
-          ncnt += 2;
-        }
+      if (ok && isfinite(r)) {
+        nsum += r;
+        ncnt += NPOL;
       }
     }
     bool all_finite = true;
@@ -1680,303 +2032,127 @@ __device__ __forceinline__ void FinalizeDistributed(const PipeParams& p, int cti
       sol[q] = nxt[q];
       all_finite = all_finite && dfinite(nxt[q]);
     }
-    WriteTables<NPOL>(p, cb, ant, s, nxt);
-    if (!all_finite) p.cb_newflag[cb] = 1u;
+    WriteTables<NPOL>(p, cb, ant, s, entry, nxt);
+    if (!all_finite) {
+      p.cb_newflag[cb] = 1u;
+      bad = true;
+    }
   };
-  // A thread's items, kFinBatch at a time: their index, slot-list and
-  // solution reads are issued together and their partial slots merged in
-  // rounds, so that the chains of dependent L2 reads of the items overlap
-  // (each item's slots are still added in slot order).
-  // Interval by interval (one round for a single interval): its items spread
-  // over all CTAs, its norm partial per CTA. An interval that has stopped
-  // keeps its solutions.
-  for (uint32_t g = 0; g < p.n_groups; ++g) {
-    nsum = 0.0;
-    ncnt = 0;
-    const bool frozen = p.n_groups > 1 && !p.host_mode &&
-                        static_cast<volatile const LoopState*>(p.state)[g].done != 0;
-    const uint32_t i_lo = p.n_groups > 1 ? p.group_cb[g] * n_items_cb : 0u;
-    const uint32_t i_hi = frozen ? i_lo : p.n_groups > 1 ? p.group_cb[g + 1] * n_items_cb : n_items;
-    constexpr int kFinBatch = 4;
-    const uint32_t item_step = gridDim.x * kPipeRuns;
-    for (uint32_t item0 = i_lo + blockIdx.x * kPipeRuns + ctid; item0 < i_hi;
-         item0 += kFinBatch * item_step) {
-      uint32_t cbv[kFinBatch], antv[kFinBatch], sv[kFinBatch], dv[kFinBatch];
-      uint32_t j0v[kFinBatch], j1v[kFinBatch], v0v[kFinBatch];
-      double2 oldv[kFinBatch][NPOL];
-  #pragma unroll
-      for (int b = 0; b < kFinBatch; ++b) {
-        const uint32_t item = item0 + b * item_step;
-        cbv[b] = antv[b] = sv[b] = dv[b] = 0;
-        j0v[b] = j1v[b] = v0v[b] = 0;
-  #pragma unroll
-        for (int q = 0; q < NPOL; ++q) oldv[b][q] = make_double2(0.0, 0.0);
-        if (item < i_hi) {
-          const uint32_t cb = item / n_items_cb;
-          const uint32_t it = item - cb * n_items_cb;
-          const uint32_t ant = it / p.n_sub;
-          const uint32_t s = it - ant * p.n_sub;
-          cbv[b] = cb;
-          antv[b] = ant;
-          sv[b] = s;
-          dv[b] = p.dir_of_sub[s];
-          j0v[b] = p.fin_off[cb * p.n_sub + s];
-          j1v[b] = p.fin_off[cb * p.n_sub + s + 1];
-          if (p.fin_first) v0v[b] = p.fin_first[cb * p.n_sub + s];
-          const double2* sol = p.solutions + size_t(item) * NPOL;
-  #pragma unroll
-          for (int q = 0; q < NPOL; ++q) oldv[b][q] = sol[q];
-        }
+  const uint32_t item_step = gridDim.x * (W * 32);
+  const uint32_t item_first =
+      (uint32_t(ctid >> 5) * gridDim.x + blockIdx.x) * 32u + uint32_t(ctid & 31);
+  struct Item {
+    uint32_t cb, ant, s;
+    uint4 list;  // FinList
+    double2 old[NPOL];
+  };
+  auto fetch = [&](uint32_t item, Item& x) {
+    x.cb = item / n_items_cb;
+    const uint32_t rem = item - x.cb * n_items_cb;
+    x.ant = rem / p.n_sub;
+    x.s = rem - x.ant * p.n_sub;
+    x.list = *reinterpret_cast<const uint4*>(p.fin_lists + x.cb * p.n_sub + x.s);
+#pragma unroll
+    for (int q = 0; q < NPOL; ++q) x.old[q] = __ldcg(sol_in + size_t(item) * NPOL + q);
+  };
+  Item x{};
+  const bool single = p.n_groups == 1;
+  // Four lanes share an item, a few slots each, where the grid has them: one
+  // round trip for 16 slots, and registers for 4 of them only.
+  const uint32_t share = single && n_items <= item_step / 4 ? 2u : 0u;
+  if (single && (item_first >> share) < n_items) fetch(item_first >> share, x);
+  if (!wait_slots()) return false;
+  // The items, warp by warp over the CTAs; a lane reads its slots of an item
+  // kR at a time and adds them in slot order, and the lanes of the item then
+  // add up theirs.
+  auto merge = [&](uint32_t item, uint32_t part) {
+    const bool range = (x.list.y & kFinRange) != 0;
+    // no partial slots to merge after the constraints
+    const uint32_t count = p.fin_mode == kFinAssignOnly ? 0u : x.list.y & ~kFinRange;
+    // the item's numerators and denominators in a partial slot (AccAdd)
+    const float* num = p.partials + size_t(x.ant) * p.acc_stride + AccNumOffset(NPOL, x.list.z, 0);
+    const float* den =
+        p.partials + size_t(x.ant) * p.acc_stride + AccDenOffset(NPOL, p.n_dir, x.list.z, 0);
+    NeumaierSum nr[NPOL], ni[NPOL], dn[NPOL];
+    constexpr uint32_t kR = 4;  // slots per round (8 at once spill the row loop)
+    for (uint32_t k = part * kR; k < count; k += kR << share) {
+      float v[kR][NPOL * 3];
+#pragma unroll
+      for (uint32_t u = 0; u < kR; ++u) {
+        if (k + u >= count) break;
+        const size_t at =
+            size_t(range ? x.list.x + k + u : p.fin_visits[x.list.x + k + u]) * p.acc_floats;
+        LoadSlot<NPOL>(num + at, den + at, v[u]);
       }
-      uint32_t n_rounds = 0;
-  #pragma unroll
-      for (int b = 0; b < kFinBatch; ++b) n_rounds = max(n_rounds, j1v[b] - j0v[b]);
-      if (p.fin_mode == kFinAssignOnly) n_rounds = 0;  // no partial slots to merge
-      NeumaierSum nr[kFinBatch][NPOL], ni[kFinBatch][NPOL], dn[kFinBatch][NPOL];
-      constexpr int kR = 4;  // slots per item and round
-      for (uint32_t k = 0; k < n_rounds; k += kR) {
-        uint32_t vis[kFinBatch][kR];
-  #pragma unroll
-        for (int b = 0; b < kFinBatch; ++b)
-  #pragma unroll
-          for (int u = 0; u < kR; ++u)
-            vis[b][u] = j0v[b] + k + u >= j1v[b] ? 0xFFFFFFFFu
-                        : p.fin_first            ? v0v[b] + k + u
-                                                 : p.fin_visits[j0v[b] + k + u];
-        float v[kFinBatch][kR][NPOL * 3];
-  #pragma unroll
-        for (int b = 0; b < kFinBatch; ++b) {
-          // the item's numerators and denominators in a partial slot (AccAdd)
-          const size_t off_n = size_t(antv[b]) * p.acc_stride + AccNumOffset(NPOL, dv[b], 0);
-          const size_t off_d =
-              size_t(antv[b]) * p.acc_stride + AccDenOffset(NPOL, p.n_dir, dv[b], 0);
-  #pragma unroll
-          for (int u = 0; u < kR; ++u) {
-            if (vis[b][u] == 0xFFFFFFFFu) continue;
-            const float* a = p.partials + size_t(vis[b][u]) * p.acc_floats;
-  #pragma unroll
-            for (int e = 0; e < NPOL * 2; ++e) v[b][u][e] = __ldcg(a + off_n + e);
-  #pragma unroll
-            for (int q = 0; q < NPOL; ++q) v[b][u][NPOL * 2 + q] = __ldcg(a + off_d + q);
-          }
-        }
-  #pragma unroll
-        for (int b = 0; b < kFinBatch; ++b)
-  #pragma unroll
-          for (int u = 0; u < kR; ++u) {
-            if (vis[b][u] == 0xFFFFFFFFu) continue;
-  #pragma unroll
-            for (int q = 0; q < NPOL; ++q) {
-              nr[b][q].Add(v[b][u][q * 2 + 0]);
-              ni[b][q].Add(v[b][u][q * 2 + 1]);
-              dn[b][q].Add(v[b][u][NPOL * 2 + q]);
-            }
-          }
-      }
-  #pragma unroll
-      for (int b = 0; b < kFinBatch; ++b) {
-        const uint32_t item = item0 + b * item_step;
-        if (item < i_hi) finish(item, cbv[b], antv[b], sv[b], oldv[b], nr[b], ni[b], dn[b]);
-      }
-    }
-    s_sum[ctid] = nsum;
-    s_cnt[ctid] = ncnt;
-    ConsumerBarrier();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (ctid < w && ctid + w < kPipeRuns) {
-        s_sum[ctid] += s_sum[ctid + w];
-        s_cnt[ctid] += s_cnt[ctid + w];
-      }
-      ConsumerBarrier();
-    }
-    if (ctid == 0) {
-      p.block_sum[size_t(g) * gridDim.x + blockIdx.x] = s_sum[0];
-      p.block_cnt[size_t(g) * gridDim.x + blockIdx.x] = s_cnt[0];
-    }
-    ConsumerBarrier();  // s_sum is reused by the next interval
-  }
-  // The last CTA finishes the iteration.
-  if (ctid == 0) {
-    __threadfence();
-    const uint32_t prev = atomicAdd(&p.counters[0], 1u);
-    *s_last = (prev == gridDim.x - 1) ? 1u : 0u;
-  }
-  ConsumerBarrier();
-  if (!*s_last) return;
-  __threadfence();
-  if (p.fin_mode == kFinStepOnly) {
-    // the assignment pass after the constraints finishes the iteration
-    if (ctid == 0) {
-      p.counters[0] = 0;
-      p.counters[2] = 0;
-    }
-    return;
-  }
-  // Channel blocks with new non-finite solutions, checked by all consumer
-  // threads at once (the serial pass below runs only when there are some).
-  uint32_t any_bad = 0;
-  if (!p.host_mode) {
-    ConsumerBarrier();  // every thread has read *s_last above
-    if (ctid == 0) *s_last = 0u;
-    ConsumerBarrier();
-    for (uint32_t cb = ctid; cb < p.n_cb; cb += kPipeRuns) {
-      const bool bad = reinterpret_cast<volatile uint32_t*>(p.cb_newflag)[cb] != 0;
-      if (!bad)
-        p.cb_flag[cb] = 0u;
-      else
-        atomicOr(s_last, 1u);
-    }
-    ConsumerBarrier();
-    any_bad = *s_last;
-  }
-  if (!p.host_mode && any_bad) {
-    // Replacement values for channel blocks with new non-finite solutions:
-    // mean |pol 0| over finite pairs; the gain tables take the replacement
-    // now, the solutions when the next finalisation reads them.
-    for (uint32_t cb = 0; cb < p.n_cb; ++cb) {
-      const bool bad = reinterpret_cast<volatile uint32_t*>(p.cb_newflag)[cb] != 0;
-      if (!bad) {
-        if (ctid == 0) p.cb_flag[cb] = 0u;
-        continue;
-      }
-      double asum = 0.0;
-      uint32_t acnt = 0;
-      for (uint32_t it = ctid; it < n_items_cb; it += kPipeRuns) {
-        const double2* sol = p.solutions + (size_t(cb) * n_items_cb + it) * NPOL;
-        bool ok = true;
-        double2 v[NPOL];
+#pragma unroll
+      for (uint32_t u = 0; u < kR; ++u) {
+        if (k + u >= count) break;
 #pragma unroll
         for (int q = 0; q < NPOL; ++q) {
-          v[q] = __ldcg(sol + q);
-          ok = ok && dfinite(v[q]);
-        }
-        if (ok) {
-          asum += hypot(v[0].x, v[0].y);
-          ++acnt;
+          nr[q].Add(v[u][q * 2 + 0]);
+          ni[q].Add(v[u][q * 2 + 1]);
+          dn[q].Add(v[u][NPOL * 2 + q]);
         }
       }
-      s_sum[ctid] = asum;
-      s_cnt[ctid] = acnt;
-      ConsumerBarrier();
-      for (int w = 128; w > 0; w >>= 1) {
-        if (ctid < w && ctid + w < kPipeRuns) {
-          s_sum[ctid] += s_sum[ctid + w];
-          s_cnt[ctid] += s_cnt[ctid + w];
-        }
-        ConsumerBarrier();
-      }
-      const double avg = s_cnt[0] == 0 ? 1.0 : s_sum[0] / double(s_cnt[0]);
-      for (uint32_t it = ctid; it < n_items_cb; it += kPipeRuns) {
-        const double2* sol = p.solutions + (size_t(cb) * n_items_cb + it) * NPOL;
-        bool ok = true;
-#pragma unroll
-        for (int q = 0; q < NPOL; ++q) ok = ok && dfinite(__ldcg(sol + q));
-        if (!ok) {
-          double2 r[NPOL];
-#pragma unroll
-          for (int q = 0; q < NPOL; ++q) r[q] = make_double2(avg, 0.0);
-          WriteTables<NPOL>(p, cb, it / p.n_sub, it % p.n_sub, r);
-        }
-      }
-      ConsumerBarrier();
-      if (ctid == 0) {
-        p.cb_avg[cb] = avg;
-        p.cb_flag[cb] = 1u;
-        p.cb_newflag[cb] = 0u;
-      }
-      ConsumerBarrier();
     }
-  }
-  if (p.n_groups > 1 && !p.host_mode) {
-    // Several intervals: one thread per interval still going sums its norm
-    // partials in CTA order and runs its control step; the loop goes on while
-    // any interval does.
-    ConsumerBarrier();  // every thread has read *s_last
-    if (ctid == 0) *s_last = 0u;
-    ConsumerBarrier();
-    const bool error = reinterpret_cast<volatile uint32_t*>(p.counters)[1] != 0;
-    for (uint32_t g = ctid; g < p.n_groups; g += kPipeRuns) {
-      LoopState& ls = p.state[g];
-      if (ls.done) continue;
-      double sum = 0.0;
-      uint64_t cnt = 0;
-      for (uint32_t b = 0; b < gridDim.x; ++b) {
-        sum += reinterpret_cast<volatile double*>(p.block_sum)[size_t(g) * gridDim.x + b];
-        cnt += reinterpret_cast<volatile uint32_t*>(p.block_cnt)[size_t(g) * gridDim.x + b];
-      }
-      bool stop = ControlStep(ls, st, sum, cnt, p.step_magnitudes + size_t(g) * p.mags_stride);
-      if (error) {
-        ls.done = 1;
-        stop = true;
-      }
-      if (!stop) atomicOr(s_last, 1u);
+    if (share) {
+      const uint32_t lanes = 15u << (ctid & 28);
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+        for (int q = 0; q < NPOL; ++q) {
+          nr[q].Join(lanes, o);
+          ni[q].Join(lanes, o);
+          dn[q].Join(lanes, o);
+        }
+      if (part) return;
     }
-    ConsumerBarrier();
+    finish(item, x.cb, x.ant, x.s, x.list.w, x.old, nr, ni, dn);
+  };
+  if (single) {
+    for (uint32_t i = item_first; (i >> share) < n_items; i += item_step) {
+      const uint32_t item = i >> share;
+      if (i != item_first) fetch(item, x);
+      merge(item, i & ((1u << share) - 1u));
+    }
+    FenceProxyAsync();  // the gain tables, before the next pass's bulk copies
+    BlockNorm<W>(ctid, nsum, ncnt, bad, s_sum, s_cnt);
     if (ctid == 0) {
-      p.counters[0] = 0;
-      p.counters[2] = 0;
-      if (p.use_handle) cudaGraphSetConditional(p.handle, *s_last ? 1u : 0u);
+      __stcg(p.block_sum + blockIdx.x, nsum);
+      __stcg(p.block_cnt + blockIdx.x, ncnt);
     }
-    return;
+    return true;
   }
-  // The per-CTA norm partials, summed by all consumer threads of the last CTA
-  // in a fixed tree order (a serial sum by one thread sat on the critical
-  // path of every iteration).
-  {
-    double sum_t = 0.0;
-    uint32_t cnt_t = 0;
-    for (uint32_t b = ctid; b < gridDim.x; b += kPipeRuns) {
-      sum_t += reinterpret_cast<volatile double*>(p.block_sum)[b];
-      cnt_t += reinterpret_cast<volatile uint32_t*>(p.block_cnt)[b];
+  // Several intervals: an interval that has stopped keeps its solutions.
+  for (uint32_t c = uint32_t(ctid >> 5) * gridDim.x + blockIdx.x; c < p.n_chunks;
+       c += gridDim.x * W) {
+    const uint2 chunk = p.chunks[c];
+    if (!p.host_mode &&
+        static_cast<volatile const LoopState*>(p.state)[chunk.y & 0xFFFFFFu].done != 0)
+      continue;
+    nsum = 0.0;
+    ncnt = 0;
+    if (uint32_t(ctid & 31) < chunk.y >> 24) {
+      const uint32_t item = chunk.x + uint32_t(ctid & 31);
+      fetch(item, x);
+      merge(item, 0);
     }
-    s_sum[ctid] = sum_t;
-    s_cnt[ctid] = cnt_t;
-    ConsumerBarrier();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (ctid < w && ctid + w < kPipeRuns) {
-        s_sum[ctid] += s_sum[ctid + w];
-        s_cnt[ctid] += s_cnt[ctid + w];
-      }
-      ConsumerBarrier();
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      nsum += __shfl_xor_sync(0xFFFFFFFFu, nsum, o);
+      ncnt += __shfl_xor_sync(0xFFFFFFFFu, ncnt, o);
+    }
+    if ((ctid & 31) == 0) {
+      __stcg(p.block_sum + c, nsum);
+      __stcg(p.block_cnt + c, ncnt);
     }
   }
-  if (ctid != 0) return;
-  const double sum = s_sum[0];
-  const uint64_t cnt = s_cnt[0];
-  p.counters[0] = 0;
-  p.counters[2] = 0;
-  if (p.host_mode) return;
-  LoopState& ls = *p.state;
-  const double mag = cnt == 0 ? 0.0 : sum / st.step_size / double(cnt);
-  const uint32_t itn = ls.iteration + 1;
-  ls.iteration = itn;
-  if (itn <= st.hard_cap) p.step_magnitudes[itn - 1] = mag;
-  const bool converged = mag <= st.accuracy;
-  bool stalled = false;
-  if (st.detect_stalling) {
-    if (itn == 1) {
-      ls.n_var_count = 1;
-      ls.step_mean = mag;
-      ls.step_var = 0.0;
-    } else {
-      ls.n_var_count += 1;
-      const double delta_1 = mag - ls.step_mean;
-      ls.step_mean += delta_1 / double(ls.n_var_count);
-      const double delta_2 = mag - ls.step_mean;
-      ls.step_var += delta_1 * delta_2;
-    }
-    if (itn >= 30)
-      stalled = ls.step_mean <
-                st.step_diff_sigma * sqrt(ls.step_var / double(ls.n_var_count));
-  }
-  const bool ready = itn >= st.max_iterations || converged || stalled;
-  const bool error = p.counters[1] != 0;
-  const bool stop =
-      (itn >= st.min_iterations && ready) || itn >= st.hard_cap || error;
-  ls.has_converged = converged;
-  ls.has_stalled = stalled;
-  ls.done = stop;
-  if (p.use_handle) cudaGraphSetConditional(p.handle, stop ? 0u : 1u);
+  FenceProxyAsync();
+  nsum = 0.0;
+  ncnt = 0;
+  BlockNorm<W>(ctid, nsum, ncnt, bad, s_sum, s_cnt);
+  return true;
 }
 
 // Builds the FP32 gain tables from the FP64 solutions: one thread per
@@ -2014,15 +2190,14 @@ struct PowerTile {
 };
 
 template <int NCORR>
-__global__ void __launch_bounds__(kPipeRuns) power_kernel(const SlabDesc* __restrict__ slabs,
-                                                          const PowerTile* __restrict__ tiles,
-                                                          uint32_t n_dir, uint32_t power_floats,
-                                                          float* __restrict__ powers) {
+__global__ void __launch_bounds__(kWarps * 32)
+    power_kernel(const SlabDesc* __restrict__ slabs, const PowerTile* __restrict__ tiles,
+                 uint32_t n_dir, uint32_t power_floats, float* __restrict__ powers) {
   const uint32_t tile = blockIdx.x / n_dir;
   const uint32_t k = blockIdx.x - tile * n_dir;
   const PowerTile t = tiles[tile];
   const SlabDesc sl = slabs[t.slab];
-  const uint32_t r = threadIdx.x;
+  const uint32_t r = threadIdx.x;  // blockDim.x: the runs of a full tile
   double q[NCORR];
 #pragma unroll
   for (int c = 0; c < NCORR; ++c) q[c] = 0.0;
@@ -2039,54 +2214,290 @@ __global__ void __launch_bounds__(kPipeRuns) power_kernel(const SlabDesc* __rest
       }
     }
   }
-  float* out = powers + size_t(tile) * power_floats + size_t(k) * NCORR * kPipeRuns;
+  float* out = powers + size_t(tile) * power_floats + (size_t(k) * blockDim.x + r) * NCORR;
 #pragma unroll
-  for (int c = 0; c < NCORR; ++c) out[c * kPipeRuns + r] = float(q[c]);
+  for (int c = 0; c < NCORR; ++c) out[c] = float(q[c]);
 }
 
-// NG lanes per run (1, 2 or 4): a tile has kPipeRuns / NG runs and lane g of a
-// run owns directions g, g + NG, ... (DMAX of them); the residual is the sum
-// over the run's lanes (warp shuffles). NG = 1: one run per lane, exactly DMAX
-// directions.
-template <int NCORR, int NPOL, int DMAX, int NG>
-__global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const PipeParams p) {
-  static_assert(kPipeRuns % NG == 0 && 32 % NG == 0, "lanes per run must divide a warp");
-  static_assert(NG == 1 || NCORR == 2, "lane groups are laid out for two correlations");
-  constexpr int RUNS = kPipeRuns / NG;  // runs per tile
-  // An unrolled graph body launches the kernel more than once per loop test:
-  // a launch after the loop has stopped does nothing.
-  if (!p.host_mode && p.use_handle) {
+// The end of a pass of pipe_kernel, from the partial slots of this CTA on;
+// false when the launch ends with it.
+template <int W, int NPOL>
+__device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
+  const int ctid = FreshTid();
+  PipeShared& sh = *SharedPtr<PipeShared>(smem_at);
+  const PipeParams& p = sh.params;
+  const bool control = !p.host_mode && p.fin_mode == kFinFused;
+  const bool is_control = blockIdx.x == gridDim.x - 1;
+  // Grid barrier: every CTA has flushed every partial slot (the launch is
+  // cooperative, so all CTAs are resident). Thread 0 polls the arrival count
+  // and passes it on through an mbarrier (a named barrier after one warp's
+  // polling loop was measured to let the other warps through early). Bounded:
+  // a timeout flags an error and the finalisation goes ahead on whatever is
+  // there; an error anywhere ends every wait.
+  // A pass may have begun before the verdict on the one before it was known
+  // (see below): if that ends the solve, the pass ends here, with nothing but
+  // partial slots written.
+  ConsumerBarrier<W>();  // this CTA's slots are written
+  if (ctid == 0) {
+    __threadfence();
+    atomicAdd(&p.counters[kCntArrive], 1u);
+  }
+  bool bad;
+  const bool go = FinalizeDistributed<W, NPOL>(p, it, ctid, sh.sum, sh.cnt, bad, [&]() {
+    if (ctid == 0) {
+      const uint32_t target = (it + 1) * gridDim.x;
+      GridWait(p.counters,
+               [&]() { return LoadAcquire(&p.counters[kCntArrive]) - sh.arrive0 >= target; });
+      if (control && it > 0) {
+        const bool known = GridWait(
+            p.counters, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it; });
+        uint32_t v = kVerdictStop;
+        if (known) v = static_cast<volatile uint32_t*>(p.counters)[kCntVerdict];
+        sh.verdict = v;
+        if (v & kVerdictStop) {
+          sh.stop = 1u;
+          __threadfence_block();
+          sh.passes = 0xFFFFFFFFu;
+        }
+      }
+      MbarArrive(&sh.flushed);
+    }
+    PipeWait(&sh.flushed, it & 1u, &sh.err, &p.counters[kCntError]);
+    return sh.stop == 0u;
+  });
+  if (!go) return false;
+  // The solutions and gain tables of every CTA are final when all have
+  // arrived; the last CTA (with the fewest rows) runs the control step. The
+  // next pass begins at once where the solve is not about to end (or its
+  // verdict could change what the pass reads: several intervals, non-finite
+  // solutions); the verdict is looked at before its finalisation, the first
+  // step that could not be undone.
+  bool all_bad = false;
+  if (ctid == 0) {
+    __threadfence();
+    atomicAdd(reinterpret_cast<unsigned long long*>(p.counters + kCntFinal),
+              1ull | (bad ? 1ull << 32 : 0ull));
+    uint64_t count = 0;
+    const uint32_t target = (it + 1) * gridDim.x;
+    const bool done = GridWait(p.counters, [&]() {
+      count = LoadAcquire64(reinterpret_cast<const uint64_t*>(p.counters + kCntFinal));
+      return uint32_t(count) - sh.final0 >= target;
+    });
+    all_bad = uint32_t(count >> 32) != sh.bad_seen;
+    sh.bad_seen = uint32_t(count >> 32);
+    if (!done) sh.stop = 1u;
+    sh.flag[1] = all_bad ? 1u : 0u;
+  }
+  if (control && is_control) {
+    ConsumerBarrier<W>();
+    const uint32_t v = ControlPass<W, NPOL>(p, ctid, sh.flag[1] != 0, sh.sum, sh.cnt, sh.flag);
+    if (ctid == 0) {
+      p.counters[kCntVerdict] = v;
+      StoreRelease(&p.counters[kCntEpoch], sh.epoch0 + it + 1);
+    }
+  }
+  if (it + 1 == p.n_iters) return false;
+  if (ctid == 0) {
+    if (control && (it == 0 || all_bad || p.n_groups > 1 || (sh.verdict & kVerdictNear))) {
+      const bool known = GridWait(
+          p.counters, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it + 1; });
+      uint32_t v = kVerdictStop;
+      if (known) v = static_cast<volatile uint32_t*>(p.counters)[kCntVerdict];
+      sh.verdict = v;
+      if (v & kVerdictStop) sh.stop = 1u;
+    }
+    __threadfence_block();
+    sh.passes = it + 1;
+    MbarArrive(&sh.ready);
+  }
+  return PipeWait(&sh.ready, it & 1u, &sh.err, &p.counters[kCntError]) && sh.stop == 0u;
+}
+
+// What a tile's fragments need of its runs besides the visibilities, one
+// block of 32-bit words per tile (equal tiles of different channel blocks
+// share one), copied to shared memory with a fragment's first row:
+//   [0] antennas of the tile, [1] first word of their list, [2] of the entries
+//   [4 ..) antenna1 | antenna2 << 16 of each run
+//   list: antenna | first entry << 16, ascending, and one end mark
+//   entries: run | side << 15 | other antenna << 16, by antenna, runs ascending
+//   (side 1: the antenna is the run's antenna 2)
+constexpr uint32_t kMetaRuns = 4;
+__host__ __device__ constexpr uint32_t MetaWords(uint32_t runs, uint32_t n_ant) {
+  const uint32_t present = n_ant < 2 * runs ? n_ant : 2 * runs;
+  return kMetaRuns + ((runs + 3u) & ~3u) + ((present + 1u + 3u) & ~3u) + ((2 * runs + 3u) & ~3u);
+}
+
+// The second half of a tile's reduction (GatherTile): one antenna's sums over
+// `n` of its entries in a tile (at most kGather) for the staged directions
+// j, j + step, ...
+constexpr uint32_t kGather = 4;
+template <int NCORR, int NPOL, int RUNS, bool HAS_Q>
+__device__ __forceinline__ void GatherEntries(const uint32_t (&en)[kGather], uint32_t n,
+                                              uint32_t gtab_at, uint32_t gain_bytes,
+                                              uint32_t stg_at, uint32_t q_at, float* row,
+                                              uint32_t n_dir, uint32_t d0, uint32_t j,
+                                              uint32_t step, uint32_t n_staged) {
+  uint32_t gains[kGather], run[kGather];
+#pragma unroll
+  for (uint32_t u = 0; u < kGather; ++u) {
+    run[u] = en[u] & 0x7FFFu;
+    gains[u] = gtab_at + (en[u] >> 16) * gain_bytes + d0 * NPOL * 8;
+  }
+#pragma unroll 2
+  for (; j < n_staged; j += step) {
+    float2 num[NPOL];
+    float den[NPOL];
+#pragma unroll
+    for (int q = 0; q < NPOL; ++q) {
+      num[q] = make_float2(0.f, 0.f);
+      den[q] = 0.f;
+    }
+    if constexpr (NPOL == 1) {
+      // one gain for every correlation: their sums are staged
+      const float4* const v_at = SharedPtr<const float4>(stg_at + j * (RUNS * 16));
+#pragma unroll
+      for (uint32_t u = 0; u < kGather; ++u) {
+        if (u >= n) break;
+        const float2 gc = *SharedPtr<const float2>(gains[u] + j * 8);
+        const float4 v = v_at[run[u]];
+        const float vy = __uint_as_float(__float_as_uint(v.y) ^ ((en[u] << 16) & 0x80000000u));
+        num[0].x = fmaf(gc.x, v.x, fmaf(-gc.y, vy, num[0].x));
+        num[0].y = fmaf(gc.x, vy, fmaf(gc.y, v.x, num[0].y));
+        den[0] = fmaf(cnorm(gc), v.z, den[0]);
+      }
+    } else {
+      const uint32_t p_at = stg_at + j * (RUNS * NCORR * 8);
+      const uint32_t qj_at = q_at + j * (RUNS * NCORR * 4);
+#pragma unroll
+      for (uint32_t u = 0; u < kGather; ++u) {
+        if (u >= n) break;
+        const uint32_t flip = (en[u] << 16) & 0x80000000u;  // side 1: the Hermitian transpose
+        float2 gb[NPOL];
+        LoadGains<NPOL>(SharedPtr<const float2>(gains[u] + j * NPOL * 8), 0, 0, 0, gb);
+        float2 Pc[NCORR];
+        LoadVisShared<NCORR>(SharedPtr<const char>(p_at), run[u], Pc);
+#pragma unroll
+        for (int c = 0; c < NCORR; ++c)
+          Pc[c].y = __uint_as_float(__float_as_uint(Pc[c].y) ^ flip);
+        float Qc[NCORR];
+        if constexpr (HAS_Q) {
+          if constexpr (NCORR == 2) {
+            const float2 w = SharedPtr<const float2>(qj_at)[run[u]];
+            Qc[0] = w.x;
+            Qc[NCORR - 1] = w.y;
+          } else {
+            const float4 w = SharedPtr<const float4>(qj_at)[run[u]];
+            Qc[0] = w.x;
+            Qc[1] = flip ? w.z : w.y;
+            Qc[2] = flip ? w.y : w.z;
+            Qc[NCORR - 1] = w.w;
+          }
+        }
+        if constexpr (NCORR == 4) {
+          const float2 t = Pc[1];
+          Pc[1] = flip ? Pc[2] : Pc[1];
+          Pc[2] = flip ? t : Pc[2];
+        }
+#pragma unroll
+        for (int c = 0; c < NCORR; ++c) {  // num += g_b P, den += |g_b|^2 Q
+          const int q = RowPol<NCORR, NPOL>(c);
+          const float2 gc = gb[ColPol<NCORR, NPOL>(c)];
+          num[q].x = fmaf(gc.x, Pc[c].x, fmaf(-gc.y, Pc[c].y, num[q].x));
+          num[q].y = fmaf(gc.x, Pc[c].y, fmaf(gc.y, Pc[c].x, num[q].y));
+          if constexpr (HAS_Q) den[q] = fmaf(cnorm(gc), Qc[c], den[q]);
+        }
+      }
+    }
+    AccAdd<NPOL, HAS_Q>(row, n_dir, d0 + j, num, den);
+  }
+}
+
+// The second half of a tile's reduction: the antennas' sums over the staged
+// directions d0 .. d0 + n_staged - 1, P at stg[j][run][corr] and the model
+// powers at q[j][run][corr] (0: none in this fragment); for one polarization
+// their sums over the correlations at stg[j][run] as P, Q, 0. Thread (i, j0) adds up
+// antenna i (and i + (W * 32), ...) for the staged directions j0, j0 +
+// step, ..., over the antenna's entries in their order, kGather entries per
+// update of an accumulator: few barriers and read-modify-write chains,
+// whatever the order of the runs. Consecutive threads take consecutive
+// antennas, mostly of consecutive runs: distinct shared-memory banks. Out of
+// line: its registers would spill the row loop.
+template <int W, int NCORR, int NPOL, int RUNS>
+__device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, uint32_t stg_at,
+                                        uint32_t q_at, uint32_t acc_at, uint32_t ctid,
+                                        uint32_t n_dir, uint32_t d0, uint32_t n_staged,
+                                        uint32_t acc_stride, uint32_t gain_stride) {
+  const uint32_t* const meta = SharedPtr<const uint32_t>(meta_at);
+  float* const acc = SharedPtr<float>(acc_at);
+  const uint32_t n_present = meta[0];
+  const uint32_t* const list = meta + meta[1];
+  const uint32_t* const ent = meta + meta[2];
+  const uint32_t step = n_present < (W * 32) ? (W * 32) / n_present : 1u;
+  const uint32_t j = step > 1 ? ctid / n_present : 0u;
+  if (j >= step || j >= n_staged) return;
+  for (uint32_t i = ctid - j * n_present; i < n_present; i += (W * 32)) {
+    const uint32_t w0 = list[i], e1 = list[i + 1] >> 16;
+    float* const row = acc + (w0 & 0xFFFFu) * acc_stride;
+    for (uint32_t e = w0 >> 16; e < e1; e += kGather) {
+      uint32_t en[kGather];
+#pragma unroll
+      for (uint32_t u = 0; u < kGather; ++u) en[u] = ent[min(e + u, e1 - 1)];
+      if (NPOL == 1 || q_at)
+        GatherEntries<NCORR, NPOL, RUNS, true>(en, e1 - e, gtab_at, gain_stride * 8, stg_at, q_at,
+                                               row, n_dir, d0, j, step, n_staged);
+      else
+        GatherEntries<NCORR, NPOL, RUNS, false>(en, e1 - e, gtab_at, gain_stride * 8, stg_at, 0,
+                                                row, n_dir, d0, j, step, n_staged);
+    }
+  }
+}
+
+// NG lanes per run (1, 2, 4 or 8): a tile has (W * 32) / NG runs and
+// lane g of a run owns directions g, g + NG, ... (DPL of them); the residual
+// is the sum over the run's lanes (warp shuffles). NG = 1: one run per lane,
+// exactly DPL directions.
+// Bound: HBM, as long as the rows' arithmetic hides under their copies. With
+// 7 consumer warps of 255 registers (two per scheduler) a row of a
+// 62-station, 10-direction interval took 0.55 us of waiting and dependent
+// arithmetic against 0.9 us of copy, and a tile's reduction 6.8 us: at most
+// DPL = 5 directions a lane keep a thread within 128 registers, so that 15
+// warps cover each other's latencies.
+// SUMQ: the model powers are summed in the row loop (else precomputed).
+constexpr int kPairValues = 6;  // model values per lane up to which two rows fit its registers
+// Of a lane's directions, staged at a time: all, or three with more than
+// kPipeDirs2 * 4 directions (40 take 101 KB of accumulators and gains).
+__host__ __device__ constexpr int StageDirs(int warps) { return warps == kWideWarps ? 3 : 8; }
+template <int NCORR, int NPOL, int DPL, int NG, bool SUMQ, int W>
+__global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p) {
+  static_assert(32 % NG == 0, "lanes per run must divide a warp");
+  constexpr int RUNS = (W * 32) / NG;  // runs per tile
+  // A solve may be several launches (of kItersPerLaunch iterations, or the
+  // unrolled body of a constrained solve's graph): a launch after the solve
+  // has stopped does nothing.
+  if (!p.host_mode) {
     bool all_done = true;
     for (uint32_t g = 0; g < p.n_groups && all_done; ++g)
       all_done = static_cast<volatile const LoopState*>(p.state)[g].done != 0;
     if (all_done) return;
   }
   extern __shared__ __align__(128) unsigned char smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* empty = full + kPipeMaxStages;
-  uint64_t* gfull = empty + kPipeMaxStages;  // gain table buffer loaded
-  uint64_t* gfree = gfull + 2;               // gain table buffer released
-  int* s_err = reinterpret_cast<int*>(gfree + 2);
-  uint32_t* s_last = reinterpret_cast<uint32_t*>(s_err + 1);
-  double* s_sum = reinterpret_cast<double*>(smem + 256);
-  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_sum + kPipeRuns);
+  PipeShared& sh = *reinterpret_cast<PipeShared*>(smem);
+  uint64_t* full = sh.full;
+  uint64_t* empty = sh.empty;
+  uint64_t* gfull = sh.gfull;
+  uint64_t* gfree = sh.gfree;
+  uint64_t* mfree = sh.mfree;
+  volatile int* s_err = &sh.err;
   float* acc = reinterpret_cast<float*>(smem + p.off_acc);
   float2* gtab_buf = reinterpret_cast<float2*>(smem + p.off_gtab);
-  float* stg = reinterpret_cast<float*>(smem + p.off_stg);
-  uint32_t* a_cnt = reinterpret_cast<uint32_t*>(smem + p.off_cnt);
-  uint32_t* a_off = reinterpret_cast<uint32_t*>(smem + p.off_off);
-  uint32_t* t_pair = reinterpret_cast<uint32_t*>(smem + p.off_pair);
-  uint16_t* ent = reinterpret_cast<uint16_t*>(smem + p.off_ent);
-  uint32_t* s_wsum = reinterpret_cast<uint32_t*>(smem + p.off_wsum);
+  float4* stg = reinterpret_cast<float4*>(smem + p.off_stg);
+  float2* stg_q = reinterpret_cast<float2*>(smem + p.off_q);
+  uint32_t* metas = reinterpret_cast<uint32_t*>(smem + p.off_meta);
   char* stages = reinterpret_cast<char*>(smem + p.off_stages);
   constexpr uint32_t E = NCORR * 8;  // bytes per visibility
   const uint32_t acc_n = p.acc_floats;
-  // NG = 1: each instantiation serves exactly DMAX directions (no padded
-  // ones); NG > 1: up to NG * DMAX.
-  const uint32_t n_dir = NG == 1 ? uint32_t(DMAX) : p.n_dir;
-  // stage: [run antennas of the fragment, first row only][data][model 0..]
-  constexpr uint32_t kRunsBytes = RUNS * 4;
-  const uint32_t stage_bytes = kRunsBytes + (1 + n_dir) * RUNS * E;
+  const uint32_t n_dir = NG == 1 ? uint32_t(DPL) : p.n_dir;
+  const uint32_t stage_bytes = (1 + n_dir) * RUNS * E;  // data, model 0, ...
   const uint32_t table_bytes = p.table_f2 * 8;
   const uint32_t S = p.stages;
 
@@ -2096,14 +2507,30 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const PipeParams 
   if (tid == 0) {
     for (uint32_t s = 0; s < S; ++s) {
       MbarInit(&full[s], 1);
-      MbarInit(&empty[s], kPipeConsumerWarps);
+      MbarInit(&empty[s], W);
     }
     for (int b = 0; b < 2; ++b) {
       MbarInit(&gfull[b], 1);
-      MbarInit(&gfree[b], kPipeConsumerWarps);
+      MbarInit(&gfree[b], W);
+      MbarInit(&mfree[b], W);
     }
-    *s_err = 0;
-    *s_last = 0;
+    MbarInit(&sh.flushed, 1);
+    MbarInit(&sh.ready, 1);
+    sh.err = 0;
+    sh.stop = 0;
+    sh.passes = 0;
+    sh.params = p;
+    // The counters before this launch. Those of finished passes and control
+    // steps cannot move before this CTA has arrived at its first grid barrier;
+    // other CTAs may have arrived there once each already.
+    sh.epoch0 = LoadAcquire(&p.counters[kCntEpoch]);
+    const uint64_t final_now =
+        LoadAcquire64(reinterpret_cast<const uint64_t*>(p.counters + kCntFinal));
+    sh.final0 = uint32_t(final_now);
+    sh.bad_seen = uint32_t(final_now >> 32);
+    const uint32_t arrived = LoadAcquire(&p.counters[kCntArrive]);
+    sh.arrive0 = arrived - arrived % gridDim.x;
+    sh.verdict = kVerdictNear;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (p.use_handle && blockIdx.x == 0) cudaGraphSetConditional(p.handle, 0);
   }
@@ -2112,531 +2539,471 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const PipeParams 
   const uint32_t f_begin = p.cta_frag_off[blockIdx.x];
   const uint32_t f_end = p.cta_frag_off[blockIdx.x + 1];
 
-  if (warp == kPipeConsumerWarps) {
+  if (warp == W) {
     // ---------------- producer warp: one thread issues all bulk copies ----
+    // The visibilities do not depend on the solutions, so the next pass's
+    // first rows are fetched while the grid finalises this one, into the ring
+    // as its stages fall free. Only the gain tables (one per visit) wait for
+    // the pass to be finished.
     if (lane != 0) return;
-    uint32_t row = 0, nvis = 0, cur_visit = 0xFFFFFFFFu;
+    uint32_t row = 0, nvis = 0, nfrag = 0;
     uint32_t st = 0, ph = 0;  // stage of `row` and the parity of its use
     bool ok = true;
-    for (uint32_t fi = f_begin; fi < f_end && ok; ++fi) {
-      const Frag f = p.frags[fi];
-      if (FragFrozen(p, f.slab)) continue;
-      const SlabDesc sl = p.slabs[f.slab];
-      if (f.visit != cur_visit) {  // new visit: its gain table first
+    for (uint32_t it = 0; it < p.n_iters && ok; ++it) {
+      bool tables_ready = it == 0;
+      const uint32_t row0 = row, nfrag0 = nfrag;  // first row and fragment of the pass
+      uint32_t cur_visit = 0xFFFFFFFFu;
+      uint32_t pending = 0xFFFFFFFFu;  // gain table not asked for yet
+      // The pending gain table, once the solutions of the pass are final;
+      // false when the launch ends instead (or a wait gave up).
+      auto fetch_table = [&]() {
+        if (!tables_ready) {
+          const uint64_t t0 = GlobalTimerNs();
+          for (uint32_t n = 1; sh.passes < it; ++n) {
+            if (*s_err) return false;
+            if ((n & 63u) == 0 && GlobalTimerNs() - t0 > kWaitBudgetNs) {
+              *s_err = 1;
+              atomicExch(&p.counters[kCntError], 1u);
+              return false;
+            }
+          }
+          if (sh.stop) return false;
+          __threadfence();
+          FenceProxyAsync();
+          tables_ready = true;
+        }
+        if (pending == 0xFFFFFFFFu) return true;
         const uint32_t b = nvis % p.n_gbuf;
         const uint32_t use = nvis / p.n_gbuf;  // earlier uses of buffer b
-        if (use >= 1 && !PipeWait(&gfree[b], (use - 1) & 1u, s_err, &p.counters[1])) {
-          ok = false;
-          break;
-        }
+        if (use >= 1 && !PipeWait(&gfree[b], (use - 1) & 1u, s_err, &p.counters[kCntError]))
+          return false;
         MbarArriveExpectTx(&gfull[b], table_bytes);
-        BulkCopyG2S(gtab_buf + size_t(b) * p.table_f2,
-                    p.tables + size_t(sl.table) * p.table_f2, table_bytes, &gfull[b]);
-        cur_visit = f.visit;
+        BulkCopyG2S(gtab_buf + size_t(b) * p.table_f2, p.tables + size_t(pending) * p.table_f2,
+                    table_bytes, &gfull[b]);
+        pending = 0xFFFFFFFFu;
         ++nvis;
-      }
-      // The fragment's tile is one tile of the packed slab: a row of it,
-      // data and all directions, is one contiguous block.
-      const uint32_t seg = (1 + n_dir) * f.n_runs * E;
-      const size_t row_step = size_t(sl.R) * (1 + n_dir) * E;
-      const char* src = static_cast<const char*>(sl.vis) + size_t(f.row_lo) * row_step +
-                        size_t(f.r0) * (1 + n_dir) * E;
-      for (uint32_t rr = f.row_lo; rr < f.row_hi; ++rr, ++row) {
-        if (row >= S && !PipeWait(&empty[st], ph ^ 1u, s_err, &p.counters[1])) {
+        return true;
+      };
+      // With several intervals the fragments of the pass depend on which
+      // intervals go on: nothing is fetched before that is known.
+      if (p.n_groups > 1 && !fetch_table()) break;
+      for (uint32_t fi = f_begin; fi < f_end && ok; ++fi) {
+        const Frag f = p.frags[fi];
+        if (FragFrozen(p, f.slab)) continue;
+        const SlabDesc sl = p.slabs[f.slab];
+        if (f.visit != cur_visit) {  // new visit: its gain table first
+          if (pending != 0xFFFFFFFFu && !fetch_table()) {
+            ok = false;
+            break;
+          }
+          pending = sl.table;
+          cur_visit = f.visit;
+          if (tables_ready && !fetch_table()) {
+            ok = false;
+            break;
+          }
+        }
+        // The fragment's tile is one tile of the packed slab: a row of it,
+        // data and all directions, is one contiguous block.
+        const uint32_t seg = (1 + n_dir) * f.n_runs * E;
+        const size_t row_step = size_t(sl.R) * (1 + n_dir) * E;
+        const char* src = static_cast<const char*>(sl.vis) + size_t(f.row_lo) * row_step +
+                          size_t(f.r0) * (1 + n_dir) * E;
+        // The next stage, free: a ring full of rows whose gain table is
+        // still pending cannot move before it.
+        auto take_stage = [&]() {
+          if (pending != 0xFFFFFFFFu && row - row0 >= S && !fetch_table()) return false;
+          return row < S || PipeWait(&empty[st], ph ^ 1u, s_err, &p.counters[kCntError]);
+        };
+        // The antenna buffer of the fragment before the last, which (like the
+        // ring) is not released before its gain table has arrived.
+        if (pending != 0xFFFFFFFFu && nfrag - nfrag0 >= 2 && !fetch_table()) {
           ok = false;
           break;
         }
-        // The fragment's run antennas travel with its first row (the run
-        // arrays are padded to whole 16-byte groups).
-        const uint32_t runs_bytes = rr == f.row_lo ? ((f.n_runs + 3u) & ~3u) * 4u : 0u;
-        MbarArriveExpectTx(&full[st], seg + runs_bytes);
-        char* dst = stages + size_t(st) * stage_bytes;
-        if (runs_bytes) BulkCopyG2S(dst, sl.run_ant + f.r0, runs_bytes, &full[st]);
-        BulkCopyG2S(dst + kRunsBytes, src, seg, &full[st]);
-        src += row_step;
-        if (++st == S) {
-          st = 0;
-          ph ^= 1u;
-        }
-      }
-      if (NG == 1 && ok && (f.flags & kFragPower)) {
-        // one more stage: the tile's model powers [dir][corr][run]
-        if (row >= S && !PipeWait(&empty[st], ph ^ 1u, s_err, &p.counters[1])) {
+        if (nfrag >= 2 && !PipeWait(&mfree[nfrag & 1u], (nfrag / 2 - 1) & 1u, s_err,
+                                    &p.counters[kCntError])) {
           ok = false;
           break;
         }
-        const uint32_t pb = n_dir * NCORR * kPipeRuns * 4;
-        MbarArriveExpectTx(&full[st], pb);
-        BulkCopyG2S(stages + size_t(st) * stage_bytes,
-                    p.powers + size_t(f.tile) * p.power_floats, pb, &full[st]);
-        ++row;
-        if (++st == S) {
-          st = 0;
-          ph ^= 1u;
+        for (uint32_t rr = f.row_lo; rr < f.row_hi; ++rr, ++row) {
+          if (!take_stage()) {
+            ok = false;
+            break;
+          }
+          // The tile's antennas travel with the fragment's first row.
+          const uint32_t mb = rr == f.row_lo ? f.meta_bytes : 0u;
+          MbarArriveExpectTx(&full[st], seg + mb);
+          if (mb) {
+            BulkCopyG2S(metas + (nfrag & 1u) * p.meta_words, p.metas + size_t(f.meta) * 4, mb,
+                        &full[st]);
+            ++nfrag;
+          }
+          BulkCopyG2S(stages + size_t(st) * stage_bytes, src, seg, &full[st]);
+          src += row_step;
+          if (++st == S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+        if (ok && (f.flags & kFragPower)) {
+          // one more stage: the tile's model powers [dir][corr][run]
+          if (!take_stage()) {
+            ok = false;
+            break;
+          }
+          const uint32_t pb = n_dir * NCORR * RUNS * 4;
+          MbarArriveExpectTx(&full[st], pb);
+          BulkCopyG2S(stages + size_t(st) * stage_bytes,
+                      p.powers + size_t(f.tile) * p.power_floats, pb, &full[st]);
+          ++row;
+          if (++st == S) {
+            st = 0;
+            ph ^= 1u;
+          }
         }
       }
+      if (ok && pending != 0xFFFFFFFFu) ok = fetch_table();
+      // a CTA without fragments still follows the passes
+      if (ok && !tables_ready) ok = fetch_table();
     }
     // Wait for the last copies, so none is in flight when the CTA ends.
     for (uint32_t k = 0; k < S && k < row; ++k) {
       const uint32_t r = row - 1 - k;
-      PipeWait(&full[r % S], (r / S) & 1u, s_err, &p.counters[1]);
+      PipeWait(&full[r % S], (r / S) & 1u, s_err, &p.counters[kCntError]);
     }
     for (uint32_t k = 0; k < p.n_gbuf && k < nvis; ++k) {
       const uint32_t v = nvis - 1 - k;
-      PipeWait(&gfull[v % p.n_gbuf], (v / p.n_gbuf) & 1u, s_err, &p.counters[1]);
+      PipeWait(&gfull[v % p.n_gbuf], (v / p.n_gbuf) & 1u, s_err, &p.counters[kCntError]);
     }
     return;
   }
 
   // ---------------- consumer warps ----------------
-  const int ctid = tid;  // 0 .. kPipeRuns - 1
-  // A warp holds 32 / NG runs; lane g * (32 / NG) + i serves run i of the
-  // warp for directions g, g + NG, ...: the 8 lanes of a quarter warp read 8
-  // consecutive runs of one direction row (distinct shared-memory banks).
-  constexpr int kRunsPerWarp = 32 / NG;
-  const int run = warp * kRunsPerWarp + lane % kRunsPerWarp;  // run within the tile
-  const int g = lane / kRunsPerWarp;  // the lane's first direction
-  const bool powers_pre = NG == 1 && p.powers != nullptr;
-  uint32_t nvis = 0, cur_visit = 0xFFFFFFFFu;
+  uint32_t nvis = 0, cur_visit = 0xFFFFFFFFu, nfrag = 0;
   uint32_t st = 0, ph = 0;  // stage of the next row and the parity of its use
   const float2* gtab = gtab_buf;
-  auto end_visit = [&]() {
-    // all consumers are done with the visit: release its gain table buffer
-    // and flush the accumulators into the visit's partial slot
-    ConsumerBarrier();
-    __syncwarp();
-    if (lane == 0) MbarArrive(&gfree[(nvis - 1) % p.n_gbuf]);
-    float* out = p.partials + size_t(cur_visit) * acc_n;
-    for (uint32_t i = ctid; i < acc_n; i += kPipeRuns) __stcg(out + i, acc[i]);
-    ConsumerBarrier();
-  };
-  // The next fragment's descriptor is fetched one fragment ahead, so that its
-  // global-memory latency overlaps the current fragment's rows; the run
-  // antennas arrive in shared memory with the fragment's first row.
-  Frag nf{};
-  if (f_begin < f_end) nf = p.frags[f_begin];
-  for (uint32_t fi = f_begin; fi < f_end; ++fi) {
-    const Frag f = nf;
-    if (fi + 1 < f_end) nf = p.frags[fi + 1];
-    if (FragFrozen(p, f.slab)) continue;
-    if (f.visit != cur_visit) {
-      if (cur_visit != 0xFFFFFFFFu) end_visit();
-      for (uint32_t i = ctid; i < acc_n; i += kPipeRuns) acc[i] = 0.f;
-      const uint32_t b = nvis % p.n_gbuf;
-      PipeWait(&gfull[b], (nvis / p.n_gbuf) & 1u, s_err, &p.counters[1]);
-      gtab = gtab_buf + size_t(b) * p.table_f2;
-      cur_visit = f.visit;
-      ++nvis;
-      ConsumerBarrier();
-    }
-    const bool active = uint32_t(run) < f.n_runs;
-    const uint32_t pitch = f.n_runs * E;  // bytes per direction row in a stage
-    const bool warp_busy = uint32_t(warp) * (32u / NG) < f.n_runs;
-    uint32_t a1 = 0, a2 = 0;
-    float2 G[DMAX][NCORR];
-    float2 P[DMAX][NCORR];
-    float Q[DMAX][NCORR];
-#pragma unroll
-    for (int k = 0; k < DMAX; ++k)
-#pragma unroll
-      for (int c = 0; c < NCORR; ++c) {
-        P[k][c] = make_float2(0.f, 0.f);
-        Q[k][c] = 0.f;
+  for (uint32_t it = 0; it < p.n_iters; ++it) {
+    // (the lane's constants, recomputed every pass: carried through the end of
+    // the pass they would spill the row loop, 0.6 us a row became 1.1 us)
+    const int ctid = FreshTid();  // 0 .. W * 32 - 1
+    const int warp = ctid >> 5, lane = ctid & 31;
+    // A warp holds 32 / NG runs; lane g * (32 / NG) + i serves run i of the
+    // warp for directions g, g + NG, ...: the 8 lanes of a quarter warp read 8
+    // consecutive runs of one direction row (NG = 8: 4 runs of two rows), in
+    // distinct shared-memory banks.
+    constexpr int kRunsPerWarp = 32 / NG;
+    const int run = warp * kRunsPerWarp + lane % kRunsPerWarp;  // run within the tile
+    const int g = lane / kRunsPerWarp;  // the lane's first direction
+    // Every lane has its first DPL - 1 directions; the last one of some lanes
+    // is past the end (n_dir > (DPL - 1) NG): they read the last direction with
+    // zero gains and drop its sums.
+    const bool last_mine = uint32_t(g + (DPL - 1) * NG) < n_dir;
+    const uint32_t last_row = min(uint32_t(g + (DPL - 1) * NG), n_dir - 1) - uint32_t(g);
+    auto end_visit = [&]() {
+      // all consumers are done with the visit: release its gain table buffer
+      // and flush the accumulators into the visit's partial slot
+      ConsumerBarrier<W>();
+      if (lane == 0) MbarArrive(&gfree[(nvis - 1) % p.n_gbuf]);
+      float4* out = reinterpret_cast<float4*>(p.partials + size_t(cur_visit) * acc_n);
+      const float4* src = reinterpret_cast<const float4*>(acc);
+      for (uint32_t i = ctid; i < acc_n / 4; i += (W * 32)) __stcg(out + i, src[i]);
+    };
+    cur_visit = 0xFFFFFFFFu;
+    for (uint32_t fi = f_begin; fi < f_end; ++fi) {
+      // (what is needed of the descriptor, read when it is: it is in L1 after
+      // the first pass, and a register held through the row loop costs more)
+      const Frag& f = p.frags[fi];
+      if (FragFrozen(p, f.slab)) continue;
+      if (f.visit != cur_visit) {
+        if (cur_visit != 0xFFFFFFFFu) {
+          end_visit();
+          ConsumerBarrier<W>();  // the accumulators are flushed
+        }
+        float4* z = reinterpret_cast<float4*>(acc);
+        for (uint32_t i = ctid; i < acc_n / 4; i += (W * 32))
+          z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t b = nvis % p.n_gbuf;
+        PipeWait(&gfull[b], (nvis / p.n_gbuf) & 1u, s_err, &p.counters[kCntError]);
+        gtab = gtab_buf + size_t(b) * p.table_f2;
+        cur_visit = f.visit;
+        ++nvis;
       }
-    for (uint32_t rr = f.row_lo; rr < f.row_hi; ++rr) {
-      const uint32_t s = st;
-      PipeWait(&full[s], ph, s_err, &p.counters[1]);
-      if (++st == S) {
-        st = 0;
-        ph ^= 1u;
+      const uint32_t* meta = metas + (nfrag & 1u) * p.meta_words;
+      const uint32_t n_runs = f.n_runs, flags = f.flags;
+      const bool active = uint32_t(run) < n_runs;
+      const bool warp_busy = uint32_t(warp) * kRunsPerWarp < n_runs;
+      // the run's data in a stage, its first direction's model, and the step
+      // to the lane's next one and to its last one
+      const uint32_t off_d = uint32_t(run) * E, pitch = n_runs * E;
+      const uint32_t off_m = off_d + (1 + g) * pitch, step_m = NG * pitch;
+      const uint32_t off_l = off_m + last_row * pitch;
+      float2 G[DPL][NCORR];
+      float2 P[DPL][NCORR];
+      float Q[SUMQ ? DPL : 1][NCORR];
+#pragma unroll
+      for (int k = 0; k < DPL; ++k)
+#pragma unroll
+        for (int c = 0; c < NCORR; ++c) {
+          P[k][c] = make_float2(0.f, 0.f);
+          if constexpr (SUMQ) Q[k][c] = 0.f;
+        }
+      const uint32_t n_rows = f.row_hi - f.row_lo;
+      PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+      if (warp_busy) {  // with the first row: the run's antennas, gain products
+        const uint32_t ap = active ? meta[kMetaRuns + run] : 0u;
+        const uint32_t a1 = ap & 0xFFFFu, a2 = ap >> 16;
+#pragma unroll
+        for (int k = 0; k < DPL; ++k) {
+          float2 ga[NPOL], gb[NPOL];
+#pragma unroll
+          for (int q = 0; q < NPOL; ++q) {
+            ga[q] = make_float2(0.f, 0.f);
+            gb[q] = make_float2(0.f, 0.f);
+          }
+          if (k < DPL - 1 || last_mine) {
+            LoadGains<NPOL>(gtab, a1, p.gain_stride, g + k * NG, ga);
+            LoadGains<NPOL>(gtab, a2, p.gain_stride, g + k * NG, gb);
+          }
+#pragma unroll
+          for (int c = 0; c < NCORR; ++c)
+            G[k][c] = cmul_conj(ga[RowPol<NCORR, NPOL>(c)], gb[ColPol<NCORR, NPOL>(c)]);
+        }
       }
-      // Warps without runs in this tile only release the stage.
-      if (warp_busy) {
-        if (rr == f.row_lo) {
-          // first row of the fragment: run antennas and the run's gain products
-          const uint32_t ap =
-              active ? reinterpret_cast<const uint32_t*>(stages + size_t(s) * stage_bytes)[run] : 0u;
-          a1 = ap & 0xFFFFu;
-          a2 = ap >> 16;
+      // NR rows at once: the dependent steps of one row (load, residual,
+      // shuffles, sums) fill the latencies of the other's.
+      auto rows = [&](auto nr) {
+        constexpr int NR = decltype(nr)::value;
+        // the model row stays in registers between the residual and the sums,
+        // or is read twice where it does not fit beside them
+        constexpr bool kKeep = DPL <= int(kPipeDirs2);
+        uint32_t stage[NR];
 #pragma unroll
-          for (int k = 0; k < DMAX; ++k) {
-            float2 ga[NPOL], gb[NPOL];
+        for (int i = 0; i < NR; ++i) {
+          PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+          stage[i] = st;
+          if (++st == S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+        // Warps without runs in this tile only release the stages.
+        if (warp_busy) {
+          // Residual R = D - sum_d G_d M_d, then P_d += R conj(M_d) and
+          // (SUMQ) Q_d += |M_d|^2. With NG > 1 each lane sums its own
+          // directions' terms and the run's lanes then add theirs up
+          // (shuffles) before D is added.
+          float2 R[NR][NCORR], M[NR][kKeep ? DPL : 1][NCORR], D[NR][NCORR];
+          auto model = [&](int i, int k, float2 (&m)[NCORR]) {
+            LoadVisShared<NCORR>(stages + stage[i] * stage_bytes +
+                                     (k < DPL - 1 ? off_m + k * step_m : off_l),
+                                 0, m);
+          };
 #pragma unroll
-            for (int q = 0; q < NPOL; ++q) {
-              ga[q] = make_float2(0.f, 0.f);
-              gb[q] = make_float2(0.f, 0.f);
+          for (int i = 0; i < NR; ++i) {
+            if constexpr (kKeep) {
+#pragma unroll
+              for (int k = 0; k < DPL; ++k) model(i, k, M[i][k]);
             }
-            const uint32_t d = g + k * NG;
-            if (d < n_dir) {
-              LoadGains<NPOL>(gtab, a1, p.gain_stride, d, ga);
-              LoadGains<NPOL>(gtab, a2, p.gain_stride, d, gb);
+            LoadVisShared<NCORR>(stages + stage[i] * stage_bytes + off_d, 0, D[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            // (in two halves, to halve the chain of dependent multiply-adds)
+            float2 h[2][NCORR];
+#pragma unroll
+            for (int c = 0; c < NCORR; ++c) {
+              h[0][c] = NG == 1 ? D[i][c] : make_float2(0.f, 0.f);
+              h[1][c] = make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < DPL; ++k) {
+              float2 m[NCORR];
+              if constexpr (kKeep) {
+#pragma unroll
+                for (int c = 0; c < NCORR; ++c) m[c] = M[i][k][c];
+              } else {
+                model(i, k, m);
+              }
+#pragma unroll
+              for (int c = 0; c < NCORR; ++c) {
+                float2& r = h[k & 1][c];
+                r.x = fmaf(-G[k][c].x, m[c].x, r.x);
+                r.x = fmaf(G[k][c].y, m[c].y, r.x);
+                r.y = fmaf(-G[k][c].x, m[c].y, r.y);
+                r.y = fmaf(-G[k][c].y, m[c].x, r.y);
+              }
             }
 #pragma unroll
             for (int c = 0; c < NCORR; ++c)
-              G[k][c] = cmul_conj(ga[RowPol<NCORR, NPOL>(c)], gb[ColPol<NCORR, NPOL>(c)]);
-          }
-        }
-        const char* base = stages + size_t(s) * stage_bytes + kRunsBytes;
-        // Residual R = D - sum_d G_d M_d, then P_d += R conj(M_d), and
-        // Q_d += |M_d|^2 unless the model powers were precomputed. The model
-        // row stays in registers between the two passes when it fits next to
-        // the accumulators (shared-memory bandwidth is the row loop's limit),
-        // else it is read from shared memory twice.
-        auto row_body = [&](auto with_q) {
-          constexpr bool kQ = decltype(with_q)::value;
-          constexpr bool kKeepM = kQ ? DMAX * NCORR <= 12 : DMAX * NCORR <= 20;
-          // The residual is summed in two halves (even and odd directions) to
-          // halve its chain of dependent multiply-adds.
-          // With NG > 1 each lane sums its own directions' terms and the
-          // run's lanes then add theirs up (shuffles) before D is added.
-          float2 Rv[NCORR], Ro[NCORR];
-          if constexpr (NG == 1) {
-            LoadVisShared<NCORR>(base, run, Rv);
-          } else {
-#pragma unroll
-            for (int c = 0; c < NCORR; ++c) Rv[c] = make_float2(0.f, 0.f);
-          }
-#pragma unroll
-          for (int c = 0; c < NCORR; ++c) Ro[c] = make_float2(0.f, 0.f);
-          float2 Mk[kKeepM ? DMAX : 1][NCORR];
-#pragma unroll
-          for (int k = 0; k < DMAX; ++k) {
-            float2 M[NCORR];
-            if (g + k * NG < int(n_dir)) {
-              LoadVisShared<NCORR>(base + size_t(1 + g + k * NG) * pitch, run, M);
-            } else {
-#pragma unroll
-              for (int c = 0; c < NCORR; ++c) M[c] = make_float2(0.f, 0.f);
-            }
-            if constexpr (kKeepM) {
-#pragma unroll
-              for (int c = 0; c < NCORR; ++c) Mk[k][c] = M[c];
-            }
-#pragma unroll
-            for (int c = 0; c < NCORR; ++c) {
-              float2& r = (k & 1) ? Ro[c] : Rv[c];
-              r.x = fmaf(-G[k][c].x, M[c].x, r.x);
-              r.x = fmaf(G[k][c].y, M[c].y, r.x);
-              r.y = fmaf(-G[k][c].x, M[c].y, r.y);
-              r.y = fmaf(-G[k][c].y, M[c].x, r.y);
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < NCORR; ++c) {
-            Rv[c].x += Ro[c].x;
-            Rv[c].y += Ro[c].y;
+              R[i][c] =
+                  DPL > 1 ? make_float2(h[0][c].x + h[1][c].x, h[0][c].y + h[1][c].y) : h[0][c];
           }
           if constexpr (NG > 1) {
 #pragma unroll
             for (int m = kRunsPerWarp; m < 32; m <<= 1)
 #pragma unroll
-              for (int c = 0; c < NCORR; ++c) {
-                Rv[c].x += __shfl_xor_sync(0xFFFFFFFFu, Rv[c].x, m);
-                Rv[c].y += __shfl_xor_sync(0xFFFFFFFFu, Rv[c].y, m);
-              }
-            float2 D[NCORR];
-            LoadVisShared<NCORR>(base, run, D);
-#pragma unroll
-            for (int c = 0; c < NCORR; ++c) {
-              Rv[c].x += D[c].x;
-              Rv[c].y += D[c].y;
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < DMAX; ++k) {
-            float2 M[NCORR];
-            if constexpr (kKeepM) {
-#pragma unroll
-              for (int c = 0; c < NCORR; ++c) M[c] = Mk[k][c];
-            } else if (g + k * NG < int(n_dir)) {
-              LoadVisShared<NCORR>(base + size_t(1 + g + k * NG) * pitch, run, M);
-            } else {
-#pragma unroll
-              for (int c = 0; c < NCORR; ++c) M[c] = make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int c = 0; c < NCORR; ++c) {
-              P[k][c].x = fmaf(Rv[c].x, M[c].x, P[k][c].x);
-              P[k][c].x = fmaf(Rv[c].y, M[c].y, P[k][c].x);
-              P[k][c].y = fmaf(Rv[c].y, M[c].x, P[k][c].y);
-              P[k][c].y = fmaf(-Rv[c].x, M[c].y, P[k][c].y);
-              if constexpr (kQ) {
-                Q[k][c] = fmaf(M[c].x, M[c].x, Q[k][c]);
-                Q[k][c] = fmaf(M[c].y, M[c].y, Q[k][c]);
-              }
-            }
-          }
-        };
-        if (powers_pre)
-          row_body(std::false_type{});
-        else
-          row_body(std::true_type{});
-      }
-      __syncwarp();
-      if (lane == 0) MbarArrive(&empty[s]);
-    }
-    if (NG == 1 && (f.flags & kFragPower)) {
-      // the tile's precomputed model powers, in the stage after its rows
-      const uint32_t s = st;
-      PipeWait(&full[s], ph, s_err, &p.counters[1]);
-      if (++st == S) {
-        st = 0;
-        ph ^= 1u;
-      }
-      if (active) {
-        const float* pw = reinterpret_cast<const float*>(stages + size_t(s) * stage_bytes);
-#pragma unroll
-        for (int k = 0; k < DMAX; ++k)
-#pragma unroll
-          for (int c = 0; c < NCORR; ++c)
-            if (k < int(n_dir)) Q[k][c] = pw[(k * NCORR + c) * kPipeRuns + ctid];
-      }
-      __syncwarp();
-      if (lane == 0) MbarArrive(&empty[s]);
-    }
-
-    // ---- tile reduction into the visit's antenna accumulators ----
-    ConsumerBarrier();  // the previous reduction is complete everywhere
-    if (f.flags & kFragDirect) {
-      // The runs form up to eight consecutive groups; within a group the
-      // first antennas are distinct and so are the second antennas. Per
-      // group, two conflict-free phases of plain shared-memory updates.
-      const uint32_t n_groups_t = (f.flags >> 8) & 0xFu;
-      uint32_t my_group = 0;
-#pragma unroll
-      for (int gi = 0; gi < int(kMaxGroups) - 1; ++gi)
-        my_group += uint32_t(run) >= ((f.group_end[gi >> 2] >> ((gi & 3) * 8)) & 0xFFu) &&
-                    uint32_t(gi + 1) < n_groups_t;
-      for (uint32_t phase = 0; phase < 2 * n_groups_t; ++phase) {
-        const int side = int(phase & 1u);
-        if (phase > 0) ConsumerBarrier();
-        if (active && my_group == (phase >> 1)) {
-          const uint32_t a = side == 0 ? a1 : a2;
-          const uint32_t b = side == 0 ? a2 : a1;
-#pragma unroll
-          for (int k = 0; k < DMAX; ++k) {
-            const uint32_t d = g + k * NG;
-            if (d < n_dir) {
-              float2 gb[NPOL];
-              LoadGains<NPOL>(gtab, b, p.gain_stride, d, gb);
-              float2 num[NPOL];
-              float den[NPOL];
-#pragma unroll
-              for (int q = 0; q < NPOL; ++q) {
-                float2 n = make_float2(0.f, 0.f);
-                float dd = 0.f;
+              for (int i = 0; i < NR; ++i)
 #pragma unroll
                 for (int c = 0; c < NCORR; ++c) {
-                  const int rp = RowPol<NCORR, NPOL>(c);
-                  const int cp = ColPol<NCORR, NPOL>(c);
-                  if (side == 0 && rp == q) {  // num += g_b P, den += |g_b|^2 Q
-                    const float2 t1 = cmul(gb[cp], P[k][c]);
-                    n.x += t1.x;
-                    n.y += t1.y;
-                    dd += cnorm(gb[cp]) * Q[k][c];
-                  }
-                  if (side == 1 && cp == q) {  // num += g_a conj(P), den += |g_a|^2 Q
-                    const float2 t2 = cmul(gb[rp], cconj(P[k][c]));
-                    n.x += t2.x;
-                    n.y += t2.y;
-                    dd += cnorm(gb[rp]) * Q[k][c];
-                  }
+                  R[i][c].x += __shfl_xor_sync(0xFFFFFFFFu, R[i][c].x, m);
+                  R[i][c].y += __shfl_xor_sync(0xFFFFFFFFu, R[i][c].y, m);
                 }
-                num[q] = n;
-                den[q] = dd;
-              }
-              AccAdd<NPOL>(acc, a, p.acc_stride, n_dir, d, num, den);
-            }
-          }
-        }
-      }
-      continue;
-    }
-    if constexpr (NG > 1) {
-      // the plan gives lane-group kernels direct tiles only
-      if (ctid == 0) atomicExch(&p.counters[1], 1u);
-      continue;
-    } else {
-    // Sorted reduction: stage the run's P/Q, counting-sort the (run, side)
-    // pairs by antenna, then (antenna, direction group) owner threads add
-    // them up; each accumulator entry has exactly one writer.
-    constexpr uint32_t NVPD = 3 * NCORR;  // staged values per direction
 #pragma unroll
-    for (int k = 0; k < DMAX; ++k) {
-      if (k < int(n_dir)) {
-#pragma unroll
-        for (int c = 0; c < NCORR; ++c) {
-          float* v = stg + ((k * NCORR + c) * 3) * kPipeRuns + ctid;
-          v[0] = P[k][c].x;
-          v[kPipeRuns] = P[k][c].y;
-          v[2 * kPipeRuns] = Q[k][c];
-        }
-      }
-    }
-    (void)NVPD;
-    t_pair[ctid] = active ? (a1 | (a2 << 16)) : 0xFFFFFFFFu;
-    for (uint32_t i = ctid; i < p.n_ant; i += kPipeRuns) a_cnt[i] = 0;
-    ConsumerBarrier();
-    // Ranks in run order (entries (run, side) of an antenna sorted by run, so
-    // that the owner's sum has a fixed order); the counts by atomics.
-    uint32_t rank1 = 0, rank2 = 0;
-    if (active) {
-      for (uint32_t j = 0; j < uint32_t(ctid); ++j) {
-        const uint32_t pr = t_pair[j];
-        if (pr == 0xFFFFFFFFu) continue;
-        const uint32_t x1 = pr & 0xFFFFu, x2 = pr >> 16;
-        rank1 += uint32_t(x1 == a1) + uint32_t(x2 == a1);
-        rank2 += uint32_t(x1 == a2) + uint32_t(x2 == a2);
-      }
-      atomicAdd(&a_cnt[a1], 1u);
-      atomicAdd(&a_cnt[a2], 1u);
-    }
-    ConsumerBarrier();
-    {
-      const uint32_t chunk = (p.n_ant + kPipeRuns - 1) / kPipeRuns;
-      const uint32_t lo = min(p.n_ant, ctid * chunk);
-      const uint32_t hi = min(p.n_ant, lo + chunk);
-      uint32_t local = 0;
-      for (uint32_t i = lo; i < hi; ++i) local += a_cnt[i];
-      uint32_t x = local;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
-      }
-      if (lane == 31) s_wsum[warp] = x;
-      ConsumerBarrier();
-      uint32_t base = 0;
-      for (int w = 0; w < warp; ++w) base += s_wsum[w];
-      uint32_t run_off = base + x - local;
-      for (uint32_t i = lo; i < hi; ++i) {
-        a_off[i] = run_off;
-        run_off += a_cnt[i];
-      }
-    }
-    ConsumerBarrier();
-    if (active) {
-      ent[a_off[a1] + rank1] = uint16_t(ctid << 1);
-      ent[a_off[a2] + rank2] = uint16_t((ctid << 1) | 1);
-    }
-    ConsumerBarrier();
-    const uint32_t n_groups = p.owner_groups;
-    for (uint32_t task = ctid; task < p.n_ant * n_groups; task += kPipeRuns) {
-      const uint32_t a = task / n_groups;
-      const uint32_t grp = task - a * n_groups;
-      const uint32_t e0 = a_off[a], e1 = e0 + a_cnt[a];
-      if (e1 == e0) continue;
-      // directions grp, grp + n_groups, ... (at most DMAX), summed in
-      // registers over the antenna's entries, then one shared update each
-      float sum[DMAX][NPOL][3];
-#pragma unroll
-      for (int i = 0; i < DMAX; ++i)
-#pragma unroll
-        for (int q = 0; q < NPOL; ++q) sum[i][q][0] = sum[i][q][1] = sum[i][q][2] = 0.f;
-      for (uint32_t e = e0; e < e1; ++e) {
-        const uint32_t en = ent[e];
-        const uint32_t j = en >> 1;
-        const bool second = (en & 1u) != 0;  // antenna a is antenna 2 of run j
-        const uint32_t pr = t_pair[j];
-        const uint32_t b = second ? (pr & 0xFFFFu) : (pr >> 16);
-#pragma unroll
-        for (int i = 0; i < DMAX; ++i) {
-          const uint32_t k = grp + i * n_groups;
-          if (k < n_dir) {
-            float2 gb[NPOL];
-            LoadGains<NPOL>(gtab, b, p.gain_stride, k, gb);
-            float2 Pc[NCORR];
-            float Qc[NCORR];
-#pragma unroll
-            for (int c = 0; c < NCORR; ++c) {
-              const float* v = stg + ((k * NCORR + c) * 3) * kPipeRuns + j;
-              Pc[c] = make_float2(v[0], v[kPipeRuns]);
-              Qc[c] = v[2 * kPipeRuns];
-            }
-#pragma unroll
-            for (int q = 0; q < NPOL; ++q) {
+            for (int i = 0; i < NR; ++i)
 #pragma unroll
               for (int c = 0; c < NCORR; ++c) {
-                const int rp = RowPol<NCORR, NPOL>(c);
-                const int cp = ColPol<NCORR, NPOL>(c);
-                if (!second && rp == q) {  // num += g_b P, den += |g_b|^2 Q
-                  const float2 t1 = cmul(gb[cp], Pc[c]);
-                  sum[i][q][0] += t1.x;
-                  sum[i][q][1] += t1.y;
-                  sum[i][q][2] += cnorm(gb[cp]) * Qc[c];
+                R[i][c].x += D[i][c].x;
+                R[i][c].y += D[i][c].y;
+              }
+          }
+#pragma unroll
+          for (int k = 0; k < DPL; ++k)
+#pragma unroll
+            for (int i = 0; i < NR; ++i) {
+              float2 mk[NCORR];
+              if constexpr (kKeep) {
+#pragma unroll
+                for (int c = 0; c < NCORR; ++c) mk[c] = M[i][k][c];
+              } else {
+                model(i, k, mk);
+              }
+#pragma unroll
+              for (int c = 0; c < NCORR; ++c) {
+                const float2 m = mk[c], r = R[i][c];
+                P[k][c].x = fmaf(r.x, m.x, P[k][c].x);
+                P[k][c].x = fmaf(r.y, m.y, P[k][c].x);
+                P[k][c].y = fmaf(r.y, m.x, P[k][c].y);
+                P[k][c].y = fmaf(-r.x, m.y, P[k][c].y);
+                if constexpr (SUMQ) {
+                  Q[k][c] = fmaf(m.x, m.x, Q[k][c]);
+                  Q[k][c] = fmaf(m.y, m.y, Q[k][c]);
                 }
-                if (second && cp == q) {  // num += g_a conj(P), den += |g_a|^2 Q
-                  const float2 t2 = cmul(gb[rp], cconj(Pc[c]));
-                  sum[i][q][0] += t2.x;
-                  sum[i][q][1] += t2.y;
-                  sum[i][q][2] += cnorm(gb[rp]) * Qc[c];
+              }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) {
+#pragma unroll
+          for (int i = 0; i < NR; ++i) MbarArrive(&empty[stage[i]]);
+        }
+      };
+      uint32_t rr = 0;
+      if constexpr (DPL * NCORR <= kPairValues)
+        if (S >= 4)  // (a shorter ring would run dry)
+          for (; rr + 2 <= n_rows; rr += 2) rows(std::integral_constant<int, 2>{});
+      for (; rr < n_rows; ++rr) rows(std::integral_constant<int, 1>{});
+
+      // ---- tile reduction into the visit's antenna accumulators ----
+      // The lanes stage their runs' sums; then one thread per (direction,
+      // antenna of the tile) adds up that antenna's runs, in the fixed order
+      // of the tile's entry list, and updates the accumulator once. Two
+      // barriers and no read-modify-write chains, whatever the runs' order.
+      uint32_t q_src = 0;  // none, or at [dir][run][corr] (SUMQ: of the staged ones)
+      uint32_t q_stage = 0;
+      if (flags & kFragPower) {
+        // the tile's precomputed model powers, in the stage after its rows
+        q_stage = st;
+        PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+        if (++st == S) {
+          st = 0;
+          ph ^= 1u;
+        }
+        q_src = SmemAddr(stages + q_stage * stage_bytes);
+      } else if (SUMQ) {
+        q_src = SmemAddr(stg_q);
+      }
+#pragma unroll
+      for (int k0 = 0; k0 < DPL; k0 += StageDirs(W)) {
+        ConsumerBarrier<W>();  // the previous reduction is complete everywhere
+        if (active) {
+#pragma unroll
+          for (int k = k0; k < DPL && k < k0 + StageDirs(W); ++k) {
+            const uint32_t j = g + (k - k0) * NG;  // staged direction k0 * NG + j
+            if (k < DPL - 1 || last_mine) {
+if constexpr (NPOL == 1) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int c = 0; c < NCORR; ++c) {
+                  v.x += P[k][c].x;
+                  v.y += P[k][c].y;
+                  if constexpr (SUMQ) v.z += Q[k][c];
+                }
+                if (!SUMQ && q_src) {
+                  const float* q =
+                      SharedPtr<const float>(q_src) + ((g + k * NG) * RUNS + run) * NCORR;
+#pragma unroll
+                  for (int c = 0; c < NCORR; ++c) v.z += q[c];
+                }
+                stg[j * RUNS + run] = v;
+              } else {
+#pragma unroll
+                for (int h = 0; h < NCORR / 2; ++h)
+                  stg[(j * RUNS + run) * (NCORR / 2) + h] = make_float4(
+                      P[k][2 * h].x, P[k][2 * h].y, P[k][2 * h + 1].x, P[k][2 * h + 1].y);
+                if constexpr (SUMQ) {
+#pragma unroll
+                  for (int h = 0; h < NCORR / 2; ++h)
+                    stg_q[(j * RUNS + run) * (NCORR / 2) + h] =
+                        make_float2(Q[k][2 * h], Q[k][2 * h + 1]);
                 }
               }
             }
           }
         }
+        ConsumerBarrier<W>();
+        const uint32_t d0 = k0 * NG;
+        const uint32_t n_staged = min(uint32_t(StageDirs(W) * NG), n_dir - d0);
+        const uint32_t q_from = q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4 : q_src;
+        GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), SmemAddr(stg), q_from,
+                                      SmemAddr(acc), ctid, n_dir, d0, n_staged, p.acc_stride,
+                                      p.gain_stride);
       }
-#pragma unroll
-      for (int i = 0; i < DMAX; ++i) {
-        const uint32_t k = grp + i * n_groups;
-        if (k < n_dir) {
-          float2 num[NPOL];
-          float den[NPOL];
-#pragma unroll
-          for (int q = 0; q < NPOL; ++q) {
-            num[q] = make_float2(sum[i][q][0], sum[i][q][1]);
-            den[q] = sum[i][q][2];
-          }
-          AccAdd<NPOL>(acc, a, p.acc_stride, n_dir, k, num, den);
-        }
-      }
-    }
-    }  // NG == 1
-  }
-  if (cur_visit != 0xFFFFFFFFu) end_visit();
-  // Grid barrier: every CTA has flushed every partial slot (the launch is
-  // cooperative, so all CTAs are resident). Every consumer warp waits on the
-  // arrival count itself (lane 0 polls, the warp follows): a named barrier
-  // after one warp's polling loop was measured to let the other warps
-  // through early. Bounded: a timeout flags an error and the finalisation
-  // goes ahead on whatever is there.
-  __threadfence();
-  ConsumerBarrier();  // this CTA's slots are written
-  if (ctid == 0) atomicAdd(&p.counters[2], 1u);
-  {
-    volatile uint32_t* arrived = &p.counters[2];
-    const uint64_t t0 = GlobalTimerNs();
-    for (uint32_t n = 1;; ++n) {
-      // lane 0 decides (all arrived, or out of time) and the warp follows
-      uint32_t stop = 0;
+      __syncwarp();
       if (lane == 0) {
-        stop = *arrived >= gridDim.x ? 1u : 0u;
-        if (!stop && (n & 63u) == 0 && GlobalTimerNs() - t0 > kWaitBudgetNs) {
-          atomicExch(&p.counters[1], 1u);
-          stop = 1u;
-        }
+        if (flags & kFragPower) MbarArrive(&empty[q_stage]);
+        MbarArrive(&mfree[nfrag & 1u]);
       }
-      if (__shfl_sync(0xFFFFFFFFu, stop, 0)) break;
-      __nanosleep(64);
+      ++nfrag;
     }
-    __threadfence();
+    if (cur_visit != 0xFFFFFFFFu) end_visit();
+    if (!EndPass<W, NPOL>(SmemAddr(smem), it)) break;
   }
-  FinalizeDistributed<NPOL>(p, ctid, s_sum, s_cnt, s_last);
 }
 
 // The assignment pass of a constrained iteration on the pipelined path
 // (fin_mode = kFinAssignOnly): FinalizeDistributed over the constrained next
-// solutions, with kPipeRuns threads per CTA (its barriers span them) and the
-// CTA count of pipe_kernel (its norm partials).
+// solutions, with kWarps warps per CTA (its barriers span them) and
+// the CTA count of pipe_kernel (its norm partials); the last CTA to arrive
+// runs the control step.
 template <int NPOL>
-__global__ void __launch_bounds__(kPipeRuns) assign_kernel(const PipeParams p) {
+__global__ void __launch_bounds__(kWarps * 32) assign_kernel(const PipeParams p) {
+  constexpr int W = kWarps;
   if (p.use_handle && static_cast<volatile const LoopState*>(p.state)->done) return;
-  __shared__ double s_sum[kPipeRuns];
-  __shared__ uint32_t s_cnt[kPipeRuns];
-  __shared__ uint32_t s_last;
-  if (threadIdx.x == 0) s_last = 0;
-  __syncthreads();
-  FinalizeDistributed<NPOL>(p, int(threadIdx.x), s_sum, s_cnt, &s_last);
+  __shared__ double s_sum[W];
+  __shared__ uint32_t s_cnt[2 * W];
+  __shared__ uint32_t s_flag[2];
+  const int ctid = int(threadIdx.x);
+  bool bad;
+  FinalizeDistributed<W, NPOL>(p, 0, ctid, s_sum, s_cnt, bad, []() { return true; });
+  auto* final = reinterpret_cast<unsigned long long*>(p.counters + kCntFinal);
+  if (ctid == 0) {
+    __threadfence();
+    const unsigned long long one = 1ull | (bad ? 1ull << 32 : 0ull);
+    const unsigned long long count = atomicAdd(final, one) + one;
+    // (a multiple of the grid between launches; the high half starts at zero)
+    s_flag[0] = uint32_t(count) % gridDim.x == 0 ? 1u : 0u;
+    s_flag[1] = uint32_t(count >> 32);
+  }
+  ConsumerBarrier<W>();
+  if (!s_flag[0]) return;
+  __threadfence();
+  const bool any_bad = s_flag[1] != 0;
+  const uint32_t v = ControlPass<W, NPOL>(p, ctid, any_bad, s_sum, s_cnt, s_flag);
+  if (ctid == 0) {
+    if (any_bad) atomicAnd(final, 0xFFFFFFFFull);
+    if (p.use_handle) cudaGraphSetConditional(p.handle, v & kVerdictStop ? 0u : 1u);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -3525,6 +3892,7 @@ void PadRuns(ChannelBlockStore& cb) {
 }
 
 using StreamFn = void (*)(StreamParams);
+struct KernelEntry;
 
 }  // namespace
 
@@ -3535,6 +3903,7 @@ struct ddsolve_ctx {
   size_t elem_bytes = 0;
   int device = 0;
   int n_sm = 0;
+  size_t max_smem = 0;  // dynamic shared memory a block may ask for
   cudaStream_t stream = nullptr;
   std::string err = "no error";
   ddsolve_settings settings{};
@@ -3583,23 +3952,23 @@ struct ddsolve_ctx {
   size_t stream_smem = 0;
   // pipelined path (pipe_kernel): chosen when eligible
   bool use_pipe = false;
+  const KernelEntry* pipe_entry = nullptr;
   const void* pipe_fn = nullptr;
   size_t pipe_smem = 0;
   uint32_t pipe_stages = 0, acc_stride = 0, gain_stride = 0;
   uint32_t pipe_ng = 1;  // lanes per run of the chosen pipe_kernel
   DevBuf d_cb_done /* new non-finite flags */, d_cb_flag, d_cb_avg, d_counters;
   DevBuf d_frags, d_cta_frag_off, d_tables, d_tab_cb, d_tab_sol, d_tab_off, d_tab_ent;
-  uint32_t n_tables = 0, table_f2 = 0, owner_groups = 1, n_gbuf = 2;
-  uint32_t off_acc = 0, off_gtab = 0, off_stg = 0, off_cnt = 0, off_off = 0,
-           off_pair = 0, off_ent = 0, off_wsum = 0, off_stages = 0;
+  uint32_t n_tables = 0, table_f2 = 0, n_gbuf = 2, meta_words = 0;
+  uint32_t off_acc = 0, off_gtab = 0, off_stg = 0, off_q = 0, off_meta = 0, off_stages = 0;
+  DevBuf d_metas;
   uint32_t n_ctas = 0, n_visits = 0, fin_blocks = 0;
   // precomputed model powers (pipe_kernel), refreshed after every upload
   bool use_powers = false, powers_dirty = true;
   uint32_t n_power_tiles = 0, power_floats = 0;
   DevBuf d_power_tiles, d_powers;
   DevBuf d_slabs, d_visits, d_cta_off, d_slab_sol, d_partials, d_fin_off,
-      d_fin_visits, d_fin_first, d_dir_of_sub, d_block_sum, d_block_cnt;
-  bool fin_ranges = false;  // pipe plan: every finalisation list is a visit range
+      d_fin_visits, d_fin_lists, d_dir_of_sub, d_block_sum, d_block_cnt;
   // solver state
   DevBuf d_sol, d_next, d_state, d_nonfinite, d_mags, d_settings;
   DevBuf d_chain;  // outputs of ddsolve_perform_iterations
@@ -3628,7 +3997,8 @@ struct ddsolve_ctx {
   std::vector<uint32_t> group_first_cb;
   uint32_t mags_stride = 1;
   DevBuf d_block_group, d_block_item0, d_block_item_end, d_group_blocks, d_cb_group;
-  DevBuf d_group_cb;  // pipe plan: first channel block of each interval, and n_cb
+  DevBuf d_chunks, d_group_chunk;  // pipe plan, several intervals (PipeParams::chunks)
+  uint32_t n_chunks = 0;
   // graph
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -3741,6 +4111,8 @@ struct KernelEntry {
   int ncorr, npol, dmax;
   const void* fn;
   int ng = 1;  // pipe_kernel: lanes per run
+  const void* fn_powers = nullptr;  // pipe_kernel: with precomputed model powers
+  int warps = 0;                    // pipe_kernel: consumer warps
 };
 
 template <int NC, int NP, int DM>
@@ -3771,70 +4143,68 @@ const KernelEntry* FindKernel(int ncorr, int npol, int need) {
   return best;
 }
 
-// Registry of pipelined-kernel instantiations keyed by (ncorr, npol, dmax).
-template <int NC, int NP, int DM>
+// Registry of pipelined-kernel instantiations keyed by (ncorr, npol,
+// directions per lane, lanes per run).
+template <int NC, int NP, int DM, int NG, int W = kWarps>
 constexpr KernelEntry PipeEntry() {
   return KernelEntry{NC, NP, DM,
-                     reinterpret_cast<const void*>(&pipe_kernel<NC, NP, DM, 1>), 1};
+                     reinterpret_cast<const void*>(&pipe_kernel<NC, NP, DM, NG, true, W>), NG,
+                     reinterpret_cast<const void*>(&pipe_kernel<NC, NP, DM, NG, false, W>), W};
 }
 
-// Lane-group variant: up to 4 * DM directions.
-template <int NC, int NP, int DM>
-constexpr KernelEntry PipeEntry4() {
-  return KernelEntry{NC, NP, DM,
-                     reinterpret_cast<const void*>(&pipe_kernel<NC, NP, DM, 4>), 4};
+template <int NC, int NP, int NG, int... DM>
+void AddPipeEntries(std::vector<KernelEntry>& k, std::integer_sequence<int, DM...>) {
+  (k.push_back(PipeEntry<NC, NP, DM + 1, NG>()), ...);
+}
+// Four lanes per run of more directions each, fewer warps.
+template <int NP, int... DM>
+void AddWideEntries(std::vector<KernelEntry>& k, std::integer_sequence<int, DM...>) {
+  (k.push_back(PipeEntry<2, NP, int(kPipeDirs2) + 1 + DM, 4, kWideWarps>()), ...);
 }
 
 const std::vector<KernelEntry>& PipeKernels() {
-  static const std::vector<KernelEntry> k = {
-      // One instantiation per direction count: a padded direction would
-      // cost a full share of the row loop, and exact counts need no guards.
-      PipeEntry<2, 2, 1>(), PipeEntry<2, 2, 2>(), PipeEntry<2, 2, 3>(),
-      PipeEntry<2, 2, 4>(), PipeEntry<2, 2, 5>(), PipeEntry<2, 2, 6>(),
-      PipeEntry<2, 2, 7>(), PipeEntry<2, 2, 8>(), PipeEntry<2, 2, 9>(),
-      PipeEntry<2, 2, 10>(), PipeEntry<2, 2, 11>(), PipeEntry<2, 2, 12>(),
-      PipeEntry<2, 1, 1>(), PipeEntry<2, 1, 2>(), PipeEntry<2, 1, 3>(),
-      PipeEntry<2, 1, 4>(), PipeEntry<2, 1, 5>(), PipeEntry<2, 1, 6>(),
-      PipeEntry<2, 1, 7>(), PipeEntry<2, 1, 8>(), PipeEntry<2, 1, 9>(),
-      PipeEntry<2, 1, 10>(), PipeEntry<2, 1, 11>(), PipeEntry<2, 1, 12>(),
-      PipeEntry<4, 2, 1>(), PipeEntry<4, 2, 2>(), PipeEntry<4, 2, 3>(),
-      PipeEntry<4, 2, 4>(),
-      PipeEntry<4, 1, 1>(), PipeEntry<4, 1, 2>(), PipeEntry<4, 1, 3>(),
-      PipeEntry<4, 1, 4>(),
-      // 13..48 directions (XX/YY): four lanes per run
-      PipeEntry4<2, 2, 4>(), PipeEntry4<2, 2, 6>(), PipeEntry4<2, 2, 8>(),
-      PipeEntry4<2, 2, 10>(), PipeEntry4<2, 2, 12>(),
-      PipeEntry4<2, 1, 4>(), PipeEntry4<2, 1, 6>(), PipeEntry4<2, 1, 8>(),
-      PipeEntry4<2, 1, 10>(), PipeEntry4<2, 1, 12>(),
-  };
+  static const std::vector<KernelEntry> k = [] {
+    std::vector<KernelEntry> v;
+    using D2 = std::make_integer_sequence<int, kPipeDirs2>;
+    using D4 = std::make_integer_sequence<int, kPipeDirs4>;
+    AddPipeEntries<2, 2, 1>(v, D2{});
+    AddPipeEntries<2, 2, 2>(v, D2{});
+    AddPipeEntries<2, 2, 4>(v, D2{});
+    AddPipeEntries<2, 1, 1>(v, D2{});
+    AddPipeEntries<2, 1, 2>(v, D2{});
+    AddPipeEntries<2, 1, 4>(v, D2{});
+    AddPipeEntries<4, 2, 1>(v, D4{});
+    AddPipeEntries<4, 2, 2>(v, D4{});
+    AddPipeEntries<4, 2, 4>(v, D4{});
+    AddPipeEntries<4, 2, 8>(v, D4{});
+    AddPipeEntries<4, 1, 1>(v, D4{});
+    AddPipeEntries<4, 1, 2>(v, D4{});
+    AddPipeEntries<4, 1, 4>(v, D4{});
+    AddPipeEntries<4, 1, 8>(v, D4{});
+    using DW = std::make_integer_sequence<int, kPipeDirsWide - kPipeDirs2>;
+    AddWideEntries<2>(v, DW{});
+    AddWideEntries<1>(v, DW{});
+    return v;
+  }();
   return k;
-}
-
-const KernelEntry* FindPipeKernel(int ncorr, int npol, int n_dir) {
-  const KernelEntry* best = nullptr;
-  for (const KernelEntry& e : PipeKernels())
-    if (e.ng == 1 && e.ncorr == ncorr && e.npol == npol && e.dmax == n_dir) best = &e;
-  if (best || std::getenv("DDSOLVE_NO_LANE_GROUPS")) return best;
-  // more directions than one lane holds: four lanes per run, the smallest
-  // instantiation with 4 * dmax >= n_dir (eight lanes per run with
-  // half-width tiles measured slower on the 40-direction interval: 418 us
-  // against 338 us per pass)
-  for (const KernelEntry& e : PipeKernels())
-    if (e.ng == 4 && e.ncorr == ncorr && e.npol == npol && 4 * e.dmax >= n_dir &&
-        (!best || e.dmax < best->dmax))
-      best = &e;
-  return best;
 }
 
 uint32_t OddAtLeast(uint32_t x) { return x | 1u; }
 
-// Strides of pipe_kernel's accumulator rows (floats; 4 mod 8, see AccAdd)
-// and gain-table rows (float2; 2 mod 4 for two polarizations, see
-// LoadGains, else odd).
+// Strides of pipe_kernel's accumulator rows (floats) and gain-table rows
+// (float2), which put consecutive antennas' entries into distinct
+// shared-memory banks: accumulators 4 mod 8 for the 16-byte updates of two
+// polarizations, 2 mod 4 for the 8-byte ones of one (AccAdd; 4 mod 8 cost
+// them two- and four-way conflicts); gains 2 mod 4 for two polarizations
+// (LoadGains), else odd.
 uint32_t PipeAccStride(uint32_t n_dir, uint32_t n_pol) {
   uint32_t s = n_dir * n_pol * 3;
-  while (s % 8 != 4) ++s;
+  while (n_pol == 2 ? s % 8 != 4 : s % 4 != 2) ++s;
   return s;
+}
+// Floats of an accumulator table and partial slot, whole 16-byte groups.
+size_t PipeAccFloats(uint32_t n_ant, uint32_t n_dir, uint32_t n_pol) {
+  return (size_t(n_ant) * PipeAccStride(n_dir, n_pol) + 3) & ~size_t(3);
 }
 uint32_t PipeGainStride(uint32_t n_dir, uint32_t n_pol) {
   uint32_t s = n_dir * n_pol;
@@ -3845,30 +4215,67 @@ uint32_t PipeGainStride(uint32_t n_dir, uint32_t n_pol) {
   return OddAtLeast(s);
 }
 
-// One pipeline stage of pipe_kernel: the fragment's run antennas (first row
-// only), then one row of data and of every direction's model.
-size_t PipeStageBytes(const ddsolve_ctx* ctx) {
-  const size_t runs = kPipeRuns / ctx->pipe_ng;
-  return runs * 4 + size_t(1 + ctx->n_dir) * runs * ctx->elem_bytes;
+// Shared memory of pipe_kernel with `ng` lanes per run: header, antenna
+// accumulators, gain tables, the staged sums of a tile (P; Q too when it is
+// summed in the row loop), two antenna buffers, the ring.
+struct PipeLayout {
+  uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
+  uint32_t meta_words;
+  uint32_t stages;  // as many as fit, 0 when not even two do
+  size_t stage_bytes;
+};
+PipeLayout MakePipeLayout(const ddsolve_ctx* ctx, uint32_t ng, uint32_t warps, uint32_t n_gbuf,
+                          bool stage_q) {
+  auto align = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
+  const size_t runs = warps * 32 / ng, n_dir = ctx->n_dir, n_corr = ctx->n_corr;
+  const size_t table_f2 =
+      (size_t(ctx->n_ant) * PipeGainStride(ctx->n_dir, ctx->n_pol) + 1) & ~size_t(1);
+  PipeLayout l{};
+  size_t off = align(sizeof(PipeShared), 128);
+  l.off_acc = uint32_t(off);
+  off += PipeAccFloats(ctx->n_ant, ctx->n_dir, ctx->n_pol) * 4;
+  l.off_gtab = uint32_t(off);
+  off += n_gbuf * table_f2 * 8;
+  l.off_stg = uint32_t(off);
+  const size_t staged = std::min<size_t>(n_dir, StageDirs(int(warps)) * ng);
+  off += staged * runs * (ctx->n_pol == 1 ? 16 : n_corr * 8);
+  l.off_q = uint32_t(off);
+  if (stage_q && ctx->n_pol != 1) off += staged * n_corr * runs * 4;
+  l.off_meta = uint32_t(off = align(off, 16));
+  l.meta_words = MetaWords(uint32_t(runs), ctx->n_ant);
+  off += 2 * size_t(l.meta_words) * 4;
+  off = align(off, 128);
+  if (off >= ctx->max_smem) return l;
+  l.off_stages = uint32_t(off);
+  l.stage_bytes = runs * (1 + n_dir) * n_corr * 8;
+  const size_t fit = (ctx->max_smem - off) / l.stage_bytes;
+  l.stages = fit < 2 ? 0u : uint32_t(std::min<size_t>(fit, kPipeMaxStages));
+  return l;
 }
 
-// Shared memory of pipe_kernel for `stages` stages, with one gain-table
-// buffer and the scratch of the sorted tile reduction (the layout is fixed in
-// BuildPipePlan, which adds the second gain-table buffer when it fits).
-size_t PipeSmemBytes(const ddsolve_ctx* ctx, uint32_t stages, uint32_t acc_stride,
-                     uint32_t gain_stride) {
-  auto align = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
-  const size_t n_ant4 = align(ctx->n_ant, 4);
-  const size_t table_f2 = (size_t(ctx->n_ant) * gain_stride + 1) & ~size_t(1);
-  size_t off = align(256 + size_t(kPipeRuns) * 12, 16);
-  off += align(size_t(ctx->n_ant) * acc_stride * 4, 16);
-  off += table_f2 * 8;
-  if (ctx->pipe_ng == 1)  // the sorted tile reduction (one run per lane only)
-    off += size_t(3) * ctx->n_corr * ctx->n_dir * kPipeRuns * 4 + 2 * n_ant4 * 4 +
-           size_t(kPipeRuns) * 4 + size_t(kPipeRuns) * 4;
-  off += 128;
-  off = align(off, 128);
-  return off + size_t(stages) * PipeStageBytes(ctx);
+// The pipe_kernel of a context: the fewest lanes per run that hold the
+// directions and leave a ring of three stages, else the deepest ring; null
+// when no variant fits. It depends on the dimensions only, so that every
+// upload packs the tiles that the plan will use. Two correlations with more
+// than 20 directions take four lanes of up to 12 directions each in the wide
+// variant: eight lanes of 5 with kWarps measured 443 us a pass against 360 for
+// 40 directions on 62 stations (twelve shuffles a row for five directions).
+const KernelEntry* FindPipeKernel(const ddsolve_ctx* ctx) {
+  const KernelEntry* best = nullptr;
+  uint32_t best_stages = 0;
+  for (uint32_t ng = 1; ng <= 8 && best_stages < 3; ng *= 2) {
+    const uint32_t dpl = (ctx->n_dir + ng - 1) / ng;
+    for (const KernelEntry& e : PipeKernels()) {
+      if (e.ncorr != int(ctx->n_corr) || e.npol != int(ctx->n_pol) || e.dmax != int(dpl) ||
+          e.ng != int(ng))
+        continue;
+      const uint32_t stages = MakePipeLayout(ctx, ng, uint32_t(e.warps), 1, true).stages;
+      if (stages <= best_stages) continue;
+      best = &e;
+      best_stages = stages;
+    }
+  }
+  return best;
 }
 
 int PreferredDirsPerLane(int ncorr) { return ncorr == 4 ? 2 : (ncorr == 2 ? 5 : 8); }
@@ -3892,16 +4299,19 @@ int CheckDims(const ddsolve_dims* dims) {
 }
 
 // Runs per tile of the packed layout: the tile of the pipelined kernel that
-// the context's correlations and direction count select (equal tiles of at
-// most kPipeRuns / NG runs, a multiple of 4, so that a tile's run antennas
-// start on a 16-byte boundary; a short remainder tile would stream its rows
-// at a fraction of the bytes per pipeline stage).
+// the context's dimensions select (equal tiles of at most its lanes / NG
+// runs, a multiple of 4; a short remainder tile would stream its rows at a
+// fraction of the bytes per pipeline stage). With eight lanes per run a
+// quarter warp reads four runs of two direction rows: their rows lie in
+// distinct shared-memory banks when the tile is 4 mod 8 runs wide.
 uint32_t LayoutTileRuns(const ddsolve_ctx* ctx, uint32_t R) {
-  const KernelEntry* e = FindPipeKernel(int(ctx->n_corr), int(ctx->n_pol), int(ctx->n_dir));
-  const uint32_t max_runs = kPipeRuns / (e ? uint32_t(e->ng) : 1u);
+  const KernelEntry* e = FindPipeKernel(ctx);
+  const uint32_t ng = e ? uint32_t(e->ng) : 1u;
+  const uint32_t max_runs = uint32_t(e ? e->warps : kWarps) * 32 / ng;
   if (R == 0) return max_runs;
   const uint32_t n_tiles = (R + max_runs - 1) / max_runs;
-  return ((R + n_tiles - 1) / n_tiles + 3u) & ~3u;
+  const uint32_t w = ((R + n_tiles - 1) / n_tiles + 3u) & ~3u;
+  return ng == 8 && w % 8 == 0 ? (w + 4 <= max_runs ? w + 4 : w - 4) : w;
 }
 
 // A point-source predict of one regular channel block (predict_kernel).
@@ -4256,15 +4666,54 @@ StageFn StagePredict(ddsolve_ctx* ctx, const ChannelBlockStore& cb, const float*
 
 constexpr int kPlanNoPipe = -1;  // BuildPipePlan: use the stream_kernel path
 
-// Plan of the pipelined path: tiles of up to kPipeRuns runs (flagged direct
-// when their first antennas are distinct and their second antennas are
-// distinct), split along their (time, channel) rows into fragments so that
-// every CTA streams the same weight of rows; visits (one partial slot each);
-// gain tables (one per channel block and solution-index vector) with the
-// lists the finalisation uses to refresh them; shared-memory layout.
+// Appends the antenna block of a tile of n runs (antenna1 | antenna2 << 16
+// each; layout at kMetaRuns) to `metas`; first = its first word / 4. `count`
+// and `at` are scratch per antenna, `count` zero between calls.
+void AppendTileMeta(std::vector<uint32_t>& metas, const uint32_t* run_ant, uint32_t n,
+                    std::vector<uint32_t>& count, std::vector<uint32_t>& at, uint32_t& first,
+                    uint32_t& bytes) {
+  std::vector<uint32_t> present;
+  for (uint32_t r = 0; r < n; ++r)
+    for (uint32_t a : {run_ant[r] & 0xFFFFu, run_ant[r] >> 16})
+      if (count[a]++ == 0) present.push_back(a);
+  std::sort(present.begin(), present.end());
+  auto pad4 = [](uint32_t x) { return (x + 3u) & ~3u; };
+  const uint32_t n_present = uint32_t(present.size());
+  const uint32_t list = kMetaRuns + pad4(n), ent = list + pad4(n_present + 1);
+  const uint32_t words = ent + pad4(2 * n);
+  const size_t base = metas.size();
+  first = uint32_t(base / 4);
+  bytes = words * 4;
+  metas.resize(base + words, 0u);
+  uint32_t* m = metas.data() + base;
+  m[0] = n_present;
+  m[1] = list;
+  m[2] = ent;
+  std::copy(run_ant, run_ant + n, m + kMetaRuns);
+  uint32_t off = 0;
+  for (uint32_t i = 0; i < n_present; ++i) {
+    m[list + i] = present[i] | (off << 16);
+    at[present[i]] = off;
+    off += count[present[i]];
+    count[present[i]] = 0;
+  }
+  m[list + n_present] = off << 16;
+  for (uint32_t r = 0; r < n; ++r) {
+    const uint32_t a1 = run_ant[r] & 0xFFFFu, a2 = run_ant[r] >> 16;
+    m[ent + at[a1]++] = r | (a2 << 16);
+    m[ent + at[a2]++] = r | 0x8000u | (a1 << 16);
+  }
+}
+
+// Plan of the pipelined path: the tiles of the packed layout with their
+// antenna blocks (TileMeta), split along their (time, channel) rows into
+// fragments so that every CTA streams the same weight of rows; visits (one
+// partial slot each); gain tables (one per channel block and solution-index
+// vector) with the lists the finalisation uses to refresh them;
+// shared-memory layout.
 int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
-                  const std::vector<uint32_t>& slab_sol, int max_optin) {
-  const uint32_t n_dir = ctx->n_dir, n_ant = ctx->n_ant, n_pol = ctx->n_pol;
+                  const std::vector<uint32_t>& slab_sol) {
+  const uint32_t n_dir = ctx->n_dir, n_ant = ctx->n_ant;
   // ---- gain tables ----
   std::map<std::vector<uint32_t>, uint32_t> table_ids;
   std::vector<uint32_t> tab_cb, tab_sol;
@@ -4295,53 +4744,47 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
 
   // ---- tiles ----
   struct Tile {
-    uint32_t slab, r0, n, rows, flags;
-    uint32_t group_end[2];
+    uint32_t slab, r0, n, rows, meta, meta_bytes;
   };
   std::vector<Tile> tiles;
-  std::vector<uint32_t> stamp1(n_ant, 0xFFFFFFFFu), stamp2(n_ant, 0xFFFFFFFFu);
-  uint32_t group_id = 0;
-  bool any_sorted = false;
+  const uint32_t tile_max = uint32_t(ctx->pipe_entry->warps) * 32 / ctx->pipe_ng;
+  std::vector<uint32_t> metas, first_tile, ant_count(n_ant, 0), ant_first(n_ant, 0);
+  uint64_t run_rows = 0, n_runs_all = 0;
   for (uint32_t gi = 0; gi < descs.size(); ++gi) {
     const SlabDesc& sd = descs[gi];
     const ChannelBlockStore& cbs = ctx->cbs[sd.cb];
     const uint32_t run_off = uint32_t(sd.run_ant - cbs.run_ant_dev.as<uint32_t>());
     // The tiles of the packed layout (LayoutTileRuns): a row of a tile is
     // one bulk copy.
-    const uint32_t max_runs = kPipeRuns / ctx->pipe_ng;
     const uint32_t tile_runs = sd.W;
-    if (tile_runs == 0 || tile_runs > max_runs || (tile_runs & 3u)) return kPlanNoPipe;
+    if (tile_runs == 0 || tile_runs > tile_max || (tile_runs & 3u)) return kPlanNoPipe;
+    // A slab whose runs are those of an earlier one (the channel blocks and
+    // time steps of a regular interval) shares its antenna blocks.
+    constexpr size_t kNone = ~size_t(0);
+    size_t like = kNone;  // its first tile
+    for (uint32_t gj = 0; gj < gi && like == kNone; ++gj) {
+      const SlabDesc& sj = descs[gj];
+      const ChannelBlockStore& cj = ctx->cbs[sj.cb];
+      const uint32_t off_j = uint32_t(sj.run_ant - cj.run_ant_dev.as<uint32_t>());
+      if (sj.R == sd.R && sj.W == sd.W &&
+          ((sj.cb == sd.cb && off_j == run_off) ||
+           std::equal(cbs.run_ant.begin() + run_off, cbs.run_ant.begin() + run_off + sd.R,
+                      cj.run_ant.begin() + off_j)))
+        like = first_tile[gj];
+      if (gj >= 8) break;  // (many unlike slabs: no point in comparing them all)
+    }
+    first_tile.push_back(uint32_t(tiles.size()));
     for (uint32_t r0 = 0; r0 < sd.R; r0 += tile_runs) {
       const uint32_t n = std::min<uint32_t>(tile_runs, sd.R - r0);
-      // Greedy split into consecutive groups whose first antennas are
-      // distinct and whose second antennas are distinct (a cyclic diagonal
-      // of the regular layout is one such group).
-      Tile t{gi, r0, n, sd.T * sd.L, 0u, {0u, 0u}};
-      uint32_t n_groups = 1;
-      ++group_id;
-      for (uint32_t r = r0; r < r0 + n; ++r) {
-        const uint32_t ap = cbs.run_ant[run_off + r];
-        const uint32_t a1 = ap & 0xFFFFu, a2 = ap >> 16;
-        if (stamp1[a1] == group_id || stamp2[a2] == group_id) {
-          if (n_groups == kMaxGroups) {
-            n_groups = kMaxGroups + 1;
-            break;
-          }
-          const uint32_t g = n_groups - 1;
-          t.group_end[g >> 2] |= (r - r0) << ((g & 3) * 8);
-          ++n_groups;
-          ++group_id;
-        }
-        stamp1[a1] = group_id;
-        stamp2[a2] = group_id;
-      }
-      if (n_groups <= kMaxGroups) {
-        const uint32_t g = n_groups - 1;
-        t.group_end[g >> 2] |= n << ((g & 3) * 8);
-        t.flags = kFragDirect | (n_groups << 8);
+      Tile t{gi, r0, n, sd.T * sd.L, 0u, 0u};
+      run_rows += uint64_t(n) * t.rows;
+      n_runs_all += n;
+      if (like != kNone) {
+        t.meta = tiles[like + r0 / tile_runs].meta;
+        t.meta_bytes = tiles[like + r0 / tile_runs].meta_bytes;
       } else {
-        t.group_end[0] = t.group_end[1] = 0;
-        any_sorted = true;
+        AppendTileMeta(metas, cbs.run_ant.data() + run_off + r0, n, ant_count, ant_first, t.meta,
+                       t.meta_bytes);
       }
       tiles.push_back(t);
     }
@@ -4349,68 +4792,65 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   // Model powers are precomputed (one stage per tile and iteration) when the
   // tiles are deep enough in rows for that stage to cost less than the two
   // multiply-adds per row, direction and correlation it replaces.
-  uint64_t run_rows = 0, n_runs_all = 0;
-  for (const Tile& t : tiles) {
-    run_rows += uint64_t(t.n) * t.rows;
-    n_runs_all += t.n;
-  }
-  if (ctx->pipe_ng > 1 && any_sorted) return kPlanNoPipe;
   const bool use_powers =
-      ctx->pipe_ng == 1 && !std::getenv("DDSOLVE_NO_POWERS") && n_runs_all > 0 &&
+      !std::getenv("DDSOLVE_NO_POWERS") && n_runs_all > 0 &&
       (ctx->tune_powers == 1 || (ctx->tune_powers < 0 && run_rows >= 16 * n_runs_all));
   // ---- fragments: rows balanced over the CTAs ----
-  // A row weighs its runs plus a fixed cost; a tile adds the cost of its
-  // reduction, about 1.25 rows per barrier phase (two per direct group; the
-  // sorted reduction as 16 phases), so that CTAs with many short tiles get
-  // fewer rows.
-  auto tile_cost = [](const Tile& t) {
-    const uint32_t phases = (t.flags & kFragDirect) ? 2u * ((t.flags >> 8) & 0xFu) : 16u;
-    return 1.25 * phases * double(t.n + 32);
-  };
+  // A row weighs its bytes; every fragment, whole tile or part of one, adds
+  // its reduction: 2.3 us against 0.7 us for a 31 KB row (62 stations, 10
+  // directions), 3.5 us where the directions are staged in two parts. The
+  // least bound under which filling the CTAs in order covers all rows is
+  // found by bisection.
+  const double reduce_bytes = ctx->pipe_entry->warps == kWideWarps ? 160e3 : 100e3;
+  auto row_cost = [&](const Tile& t) { return double(t.n) * (1 + n_dir) * ctx->elem_bytes + 1e3; };
+  auto frag_cost = [&](const Tile&) { return reduce_bytes; };
   uint64_t total_rows = 0;
-  double total_w = 0.0;
+  double total_w = 0.0, max_one = 0.0;
   for (const Tile& t : tiles) {
     total_rows += t.rows;
-    total_w += double(t.rows) * double(t.n + 32) + tile_cost(t);
+    total_w += double(t.rows) * row_cost(t) + frag_cost(t);
+    max_one = std::max(max_one, frag_cost(t) + row_cost(t));
   }
   const uint32_t max_ctas = uint32_t(ctx->n_sm);
   const uint32_t n_ctas = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(max_ctas, total_rows)));
   std::vector<Frag> frags;
   std::vector<uint32_t> cta_off(n_ctas + 1, 0);
-  {
-    double cum = 0.0;
-    uint32_t cur_cta = 0;
-    for (const Tile& t : tiles) {
-      const double w = double(t.n + 32);
-      cum += tile_cost(t);
-      uint32_t lo = 0;
-      while (lo < t.rows) {
-        // last row of this tile that stays on cur_cta
-        uint32_t hi = lo;
-        while (hi < t.rows) {
-          const double mid = cum + (double(hi - lo) + 0.5) * w;
-          uint32_t c = uint32_t(mid * n_ctas / total_w);
-          if (c >= n_ctas) c = n_ctas - 1;
-          if (c != cur_cta) break;
-          ++hi;
+  // Fills the CTAs up to `bound` each, in order; false when they do not hold
+  // all rows. With `emit` the fragments are written down.
+  auto fill = [&](double bound, bool emit) {
+    uint32_t cta = 0;
+    double used = 0.0;
+    for (uint32_t ti = 0; ti < tiles.size(); ++ti) {
+      const Tile& t = tiles[ti];
+      const double w = row_cost(t), fixed = frag_cost(t);
+      for (uint32_t lo = 0; lo < t.rows;) {
+        const double room = (bound - used - fixed) / w + 1e-6;
+        if (room < 1.0) {
+          if (++cta == n_ctas) return false;
+          if (emit) cta_off[cta] = uint32_t(frags.size());
+          used = 0.0;
+          continue;
         }
-        if (hi > lo) {
-          const uint32_t ti = uint32_t(&t - tiles.data());
-          const uint32_t fl = t.flags | (use_powers && lo == 0 ? kFragPower : 0u);
-          frags.push_back({t.slab, t.r0, t.n, fl, lo, hi, 0, ti,
-                           {t.group_end[0], t.group_end[1]}});
-          cum += double(hi - lo) * w;
-          lo = hi;
-        }
-        if (lo < t.rows) {
-          ++cur_cta;
-          cta_off[cur_cta] = uint32_t(frags.size());
-        }
+        const uint32_t n = uint32_t(std::min<double>(room, t.rows - lo));
+        if (emit)
+          frags.push_back({t.slab, t.r0, t.n, use_powers && lo == 0 ? kFragPower : 0u, lo, lo + n,
+                           0, ti, t.meta, t.meta_bytes, {0, 0}});
+        used += fixed + n * w;
+        lo += n;
       }
     }
-    for (uint32_t c = cur_cta + 1; c <= n_ctas; ++c) cta_off[c] = uint32_t(frags.size());
-    for (uint32_t c = 1; c <= n_ctas; ++c) cta_off[c] = std::max(cta_off[c], cta_off[c - 1]);
-    cta_off[n_ctas] = uint32_t(frags.size());
+    if (emit)
+      for (uint32_t c = cta + 1; c <= n_ctas; ++c) cta_off[c] = uint32_t(frags.size());
+    return true;
+  };
+  if (!tiles.empty()) {
+    double lo = std::max(max_one, total_w / n_ctas), hi = lo;
+    while (!fill(hi, false)) hi *= 1.25;
+    for (int i = 0; i < 24 && hi > lo * 1.002; ++i) {
+      const double mid = 0.5 * (lo + hi);
+      (fill(mid, false) ? hi : lo) = mid;
+    }
+    fill(hi, true);
   }
   // ---- visits ----
   uint32_t n_visits = 0;
@@ -4434,65 +4874,49 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
       if (sub < ctx->n_sub) lists[size_t(sd.cb) * ctx->n_sub + sub].push_back(v);
     }
   }
-  std::vector<uint32_t> fin_off(lists.size() + 1, 0), fin_visits;
-  for (size_t i = 0; i < lists.size(); ++i) {
-    fin_off[i] = uint32_t(fin_visits.size());
-    fin_visits.insert(fin_visits.end(), lists[i].begin(), lists[i].end());
-  }
-  fin_off[lists.size()] = uint32_t(fin_visits.size());
   // Visits are numbered in CTA order and CTAs take the slabs in order, so a
   // (channel block, sub-solution) whose slabs are consecutive has a range of
-  // visits: the finalisation then needs its first visit only.
-  bool ranges = true;
-  std::vector<uint32_t> fin_first(lists.size(), 0);
-  for (size_t i = 0; i < lists.size() && ranges; ++i) {
-    for (size_t k = 1; k < lists[i].size() && ranges; ++k)
-      ranges = lists[i][k] == lists[i][k - 1] + 1;
-    if (!lists[i].empty()) fin_first[i] = lists[i][0];
+  // visits.
+  std::vector<uint32_t> fin_visits;
+  std::vector<FinList> fin_lists(lists.size());
+  for (size_t i = 0; i < lists.size(); ++i) {
+    const std::vector<uint32_t>& l = lists[i];
+    bool range = !l.empty();
+    for (size_t k = 1; k < l.size() && range; ++k) range = l[k] == l[k - 1] + 1;
+    FinList& f = fin_lists[i];
+    f.first = range ? l[0] : uint32_t(fin_visits.size());
+    f.count = uint32_t(l.size()) | (range ? kFinRange : 0u);
+    if (!range) fin_visits.insert(fin_visits.end(), l.begin(), l.end());
+    f.dir = ctx->dir_of_sub[i % ctx->n_sub];
+    f.entry = tlists[i].size() == 1 ? tlists[i][0] : kManyEntries;
   }
-  ctx->fin_ranges = ranges;
 
   // ---- shared-memory layout ----
-  auto align = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
-  size_t off = 256 + size_t(kPipeRuns) * 12;
-  ctx->off_acc = uint32_t(align(off, 16));
-  off = ctx->off_acc + align(size_t(n_ant) * ctx->acc_stride * 4, 16);
-  ctx->off_gtab = uint32_t(off);
   // Two gain-table buffers (the next visit's table loads while the current
-  // one is in use) unless that leaves fewer than four stages.
-  {
-    const size_t stage_b = PipeStageBytes(ctx);
-    const size_t rest = size_t(3) * ctx->n_corr * n_dir * kPipeRuns * 4 + 2 * align(n_ant, 4) * 4 +
-                        size_t(kPipeRuns) * 8 + 256;
-    const size_t with2 = off + 2 * size_t(table_f2) * 8 + (any_sorted ? rest : 256);
-    ctx->n_gbuf = (with2 + 4 * stage_b <= size_t(max_optin)) ? 2u : 1u;
-    // a requested count, where two buffers still leave two stages
-    if (ctx->tune_gbuf == 1) ctx->n_gbuf = 1;
-    if (ctx->tune_gbuf == 2 && with2 + 2 * stage_b <= size_t(max_optin)) ctx->n_gbuf = 2;
+  // one is in use) unless that leaves fewer than three stages, or as asked for
+  // where two stages still fit.
+  const uint32_t warps = uint32_t(ctx->pipe_entry->warps);
+  uint32_t n_gbuf = ctx->tune_gbuf == 1 ? 1u : 2u;
+  PipeLayout lay = MakePipeLayout(ctx, ctx->pipe_ng, warps, n_gbuf, !use_powers);
+  if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 3u)) {
+    n_gbuf = 1;
+    lay = MakePipeLayout(ctx, ctx->pipe_ng, warps, n_gbuf, !use_powers);
   }
-  off += size_t(ctx->n_gbuf) * table_f2 * 8;
-  const size_t n_ant4 = align(n_ant, 4);
-  ctx->off_stg = uint32_t(off);
-  if (any_sorted) off += size_t(3) * ctx->n_corr * n_dir * kPipeRuns * 4;
-  ctx->off_cnt = uint32_t(off);
-  if (any_sorted) off += n_ant4 * 4;
-  ctx->off_off = uint32_t(off);
-  if (any_sorted) off += n_ant4 * 4;
-  ctx->off_pair = uint32_t(off);
-  if (any_sorted) off += size_t(kPipeRuns) * 4;
-  ctx->off_ent = uint32_t(off);
-  if (any_sorted) off += size_t(kPipeRuns) * 2 * 2;
-  ctx->off_wsum = uint32_t(off);
-  off += 32 * 4;
-  ctx->off_stages = uint32_t(align(off, 128));
-  const size_t stage_bytes = PipeStageBytes(ctx);
-  const size_t room = size_t(max_optin) > ctx->off_stages ? size_t(max_optin) - ctx->off_stages : 0;
-  uint32_t stages = uint32_t(std::min<size_t>(kPipeMaxStages, room / stage_bytes));
+  uint32_t stages = lay.stages;
   if (ctx->tune_stages >= 2) stages = std::min(stages, ctx->tune_stages);
   if (stages < 2)
     return ctx->Fail(DDSOLVE_E_UNSUPPORTED, "pipelined kernel does not fit in shared memory");
+  ctx->n_gbuf = n_gbuf;
+  ctx->off_acc = lay.off_acc;
+  ctx->off_gtab = lay.off_gtab;
+  ctx->off_stg = lay.off_stg;
+  ctx->off_q = lay.off_q;
+  ctx->off_meta = lay.off_meta;
+  ctx->off_stages = lay.off_stages;
+  ctx->meta_words = lay.meta_words;
   ctx->pipe_stages = stages;
-  ctx->pipe_smem = ctx->off_stages + stages * stage_bytes;
+  ctx->pipe_smem = lay.off_stages + stages * lay.stage_bytes;
+  ctx->pipe_fn = use_powers ? ctx->pipe_entry->fn_powers : ctx->pipe_entry->fn;
   DDS_CHECK_CUDA(ctx, cudaFuncSetAttribute(ctx->pipe_fn,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            int(ctx->pipe_smem)));
@@ -4500,7 +4924,6 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   ctx->n_visits = n_visits;
   ctx->n_tables = n_tables;
   ctx->table_f2 = table_f2;
-  ctx->owner_groups = std::max<uint32_t>(1u, std::min<uint32_t>(n_dir, uint32_t(kPipeRuns) / n_ant));
   const uint32_t n_items = ctx->n_cb * ctx->n_ant * ctx->n_sub;
   ctx->fin_blocks = (n_items + kThreads - 1) / kThreads;
 
@@ -4514,13 +4937,12 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   int rc;
   if ((rc = upload(ctx->d_slabs, descs.data(), descs.size() * sizeof(SlabDesc)))) return rc;
   if ((rc = upload(ctx->d_frags, frags.data(), frags.size() * sizeof(Frag)))) return rc;
+  if ((rc = upload(ctx->d_metas, metas.data(), metas.size() * 4))) return rc;
   if ((rc = upload(ctx->d_cta_frag_off, cta_off.data(), cta_off.size() * 4))) return rc;
   if ((rc = upload(ctx->d_slab_sol, slab_sol.data(), slab_sol.size() * 4))) return rc;
-  if ((rc = upload(ctx->d_fin_off, fin_off.data(), fin_off.size() * 4))) return rc;
-  if ((rc = upload(ctx->d_fin_visits, fin_visits.data(), fin_visits.size() * 4))) return rc;
-  if ((rc = upload(ctx->d_fin_first, fin_first.data(), fin_first.size() * 4))) return rc;
-  if ((rc = upload(ctx->d_dir_of_sub, ctx->dir_of_sub.data(), ctx->dir_of_sub.size() * 4)))
+  if ((rc = upload(ctx->d_fin_lists, fin_lists.data(), fin_lists.size() * sizeof(FinList))))
     return rc;
+  if ((rc = upload(ctx->d_fin_visits, fin_visits.data(), fin_visits.size() * 4))) return rc;
   if ((rc = upload(ctx->d_tab_cb, tab_cb.data(), tab_cb.size() * 4))) return rc;
   if ((rc = upload(ctx->d_tab_sol, tab_sol.data(), tab_sol.size() * 4))) return rc;
   if ((rc = upload(ctx->d_tab_off, tab_off.data(), tab_off.size() * 4))) return rc;
@@ -4528,7 +4950,7 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   ctx->use_powers = use_powers;
   ctx->powers_dirty = true;
   ctx->n_power_tiles = uint32_t(tiles.size());
-  ctx->power_floats = n_dir * ctx->n_corr * kPipeRuns;
+  ctx->power_floats = n_dir * ctx->n_corr * tile_max;
   if (use_powers) {
     std::vector<PowerTile> pt(tiles.size());
     for (size_t i = 0; i < tiles.size(); ++i) pt[i] = {tiles[i].slab, tiles[i].r0, tiles[i].n, 0u};
@@ -4539,28 +4961,38 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_tables.ptr, 0, size_t(n_tables) * table_f2 * 8,
                                       ctx->stream));
   DDS_CHECK_CUDA(ctx, ctx->d_partials.Reserve(
-                          std::max<size_t>(1, size_t(n_visits) * n_ant * ctx->acc_stride) * 4));
-  // norm partials per (interval, CTA)
+                          std::max<size_t>(1, size_t(n_visits) *
+                                                  PipeAccFloats(n_ant, n_dir, ctx->n_pol)) *
+                              4));
+  // norm partials per CTA, or per chunk of several intervals
   {
-    const size_t n_part = std::max<size_t>(size_t(n_ctas) * ctx->n_groups, ctx->fin_blocks);
+    std::vector<uint32_t> cb_group(ctx->n_cb, 0), group_chunk{0};
+    std::vector<uint2> chunks;
+    const uint32_t items_cb = n_ant * ctx->n_sub;
+    for (uint32_t g = 0; g < ctx->n_groups && ctx->n_groups > 1; ++g) {
+      const uint32_t cb0 = ctx->group_first_cb[g], cb1 = ctx->group_first_cb[g + 1];
+      for (uint32_t cb = cb0; cb < cb1; ++cb) cb_group[cb] = g;
+      for (uint32_t i = cb0 * items_cb; i < cb1 * items_cb; i += 32)
+        chunks.push_back({i, std::min(32u, cb1 * items_cb - i) << 24 | g});
+      group_chunk.push_back(uint32_t(chunks.size()));
+    }
+    ctx->n_chunks = uint32_t(chunks.size());
+    const size_t n_part = std::max<size_t>(std::max<size_t>(n_ctas, chunks.size()), ctx->fin_blocks);
     DDS_CHECK_CUDA(ctx, ctx->d_block_sum.Reserve(n_part * 8));
     DDS_CHECK_CUDA(ctx, ctx->d_block_cnt.Reserve(n_part * 4));
-    std::vector<uint32_t> cb_group(ctx->n_cb, 0), group_cb(ctx->n_groups + 1, 0);
-    for (uint32_t g = 0; g < ctx->n_groups; ++g) {
-      group_cb[g] = ctx->n_groups == 1 ? 0u : ctx->group_first_cb[g];
-      group_cb[g + 1] = ctx->n_groups == 1 ? ctx->n_cb : ctx->group_first_cb[g + 1];
-      for (uint32_t cb = group_cb[g]; cb < group_cb[g + 1]; ++cb) cb_group[cb] = g;
-    }
     if ((rc = upload(ctx->d_cb_group, cb_group.data(), cb_group.size() * 4))) return rc;
-    if ((rc = upload(ctx->d_group_cb, group_cb.data(), group_cb.size() * 4))) return rc;
+    if ((rc = upload(ctx->d_chunks, chunks.data(), chunks.size() * sizeof(uint2)))) return rc;
+    if ((rc = upload(ctx->d_group_chunk, group_chunk.data(), group_chunk.size() * 4))) return rc;
+    // the copies read these vectors until the stream is synchronised
+    DDS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
   DDS_CHECK_CUDA(ctx, ctx->d_cb_done.Reserve(size_t(ctx->n_cb) * 4));
   DDS_CHECK_CUDA(ctx, ctx->d_cb_flag.Reserve(size_t(ctx->n_cb) * 4));
   DDS_CHECK_CUDA(ctx, ctx->d_cb_avg.Reserve(size_t(ctx->n_cb) * 8));
-  DDS_CHECK_CUDA(ctx, ctx->d_counters.Reserve(16));
+  DDS_CHECK_CUDA(ctx, ctx->d_counters.Reserve(kCounterBytes));
   DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_done.ptr, 0, size_t(ctx->n_cb) * 4, ctx->stream));
   DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_flag.ptr, 0, size_t(ctx->n_cb) * 4, ctx->stream));
-  DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+  DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
   DDS_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->plan_dirty = false;
   ctx->DestroyGraph();
@@ -4696,42 +5128,22 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   ctx->pipe_ng = 1;
   if (allow_pipe && ctx->tune_ng == 0 && ctx->tune_pipe != 0 &&
       (ctx->n_corr == 2 || ctx->n_corr == 4) && !std::getenv("DDSOLVE_NO_PIPE")) {
-    const KernelEntry* pe =
-        FindPipeKernel(int(ctx->n_corr), int(ctx->n_pol), int(ctx->n_dir));
-    if (pe) ctx->pipe_ng = uint32_t(pe->ng);
-    const uint32_t acc_stride = PipeAccStride(ctx->n_dir, ctx->n_pol);
-    const uint32_t gain_stride = PipeGainStride(ctx->n_dir, ctx->n_pol);
-    uint32_t stages = 0;
-    for (uint32_t st = kPipeMaxStages; st >= 2 && pe; --st)
-      if (PipeSmemBytes(ctx, st, acc_stride, gain_stride) <= size_t(max_optin)) {
-        stages = st;
-        break;
-      }
-    if (pe && stages >= 2) {
-      const size_t smem = PipeSmemBytes(ctx, stages, acc_stride, gain_stride);
-      DDS_CHECK_CUDA(ctx, cudaFuncSetAttribute(
-                              pe->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(smem)));
-      int occ = 0;
-      DDS_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                              &occ, pe->fn, kPipeThreads, smem));
-      if (occ >= 1) {
-        ctx->use_pipe = true;
-        ctx->pipe_fn = pe->fn;
-        ctx->pipe_smem = smem;
-        ctx->pipe_stages = stages;
-        ctx->acc_stride = acc_stride;
-        ctx->gain_stride = gain_stride;
-        ctx->dmax = uint32_t(pe->dmax);
-        ctx->ng = 1;
-      }
+    const KernelEntry* pe = FindPipeKernel(ctx);
+    if (pe) {
+      ctx->use_pipe = true;
+      ctx->pipe_entry = pe;
+      ctx->pipe_ng = uint32_t(pe->ng);
+      ctx->acc_stride = PipeAccStride(ctx->n_dir, ctx->n_pol);
+      ctx->gain_stride = PipeGainStride(ctx->n_dir, ctx->n_pol);
+      ctx->dmax = uint32_t(pe->dmax);
+      ctx->ng = 1;
     }
   }
   int occ = 1;
   size_t slot_floats = 0;
   uint32_t runs_per_block = 0;
   if (ctx->use_pipe) {
-    runs_per_block = kPipeRuns;
+    runs_per_block = uint32_t(ctx->pipe_entry->warps) * 32 / ctx->pipe_ng;
     slot_floats = size_t(ctx->n_ant) * ctx->acc_stride;
   } else {
     // Kernel choice: ng lanes per run so that each lane handles at most the
@@ -4809,7 +5221,7 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
       }
     }
   }
-  if (ctx->use_pipe) return BuildPipePlan(ctx, descs, slab_sol, max_optin);
+  if (ctx->use_pipe) return BuildPipePlan(ctx, descs, slab_sol);
   ctx->pipe_ng = 1;
   const uint32_t max_ctas = uint32_t(ctx->n_sm) * uint32_t(occ);
   uint32_t n_ctas = std::max<uint32_t>(1, std::min<uint32_t>(max_ctas, uint32_t(steps.size())));
@@ -4914,12 +5326,12 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   DDS_CHECK_CUDA(ctx, ctx->d_cb_done.Reserve(size_t(ctx->n_cb) * 4));
   DDS_CHECK_CUDA(ctx, ctx->d_cb_flag.Reserve(size_t(ctx->n_cb) * 4));
   DDS_CHECK_CUDA(ctx, ctx->d_cb_avg.Reserve(size_t(ctx->n_cb) * 8));
-  DDS_CHECK_CUDA(ctx, ctx->d_counters.Reserve(16));
+  DDS_CHECK_CUDA(ctx, ctx->d_counters.Reserve(kCounterBytes));
   DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_done.ptr, 0, size_t(ctx->n_cb) * 4,
                                       ctx->stream));
   DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_flag.ptr, 0, size_t(ctx->n_cb) * 4,
                                       ctx->stream));
-  DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+  DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
   DDS_CHECK_CUDA(ctx, ctx->d_partials.Reserve(
                           std::max<size_t>(1, size_t(ctx->n_visits) * slot_floats) * 4));
   const size_t n_block_partials = std::max<size_t>(ctx->fin_blocks, ctx->n_ctas);
@@ -5006,28 +5418,26 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.acc_stride = ctx->acc_stride;
   p.gain_stride = ctx->gain_stride;
   p.stages = ctx->pipe_stages;
-  p.acc_floats = ctx->n_ant * ctx->acc_stride;
-  p.owner_groups = ctx->owner_groups;
+  p.acc_floats = uint32_t(PipeAccFloats(ctx->n_ant, ctx->n_dir, ctx->n_pol));
+  p.metas = ctx->d_metas.as<uint32_t>();
+  p.meta_words = ctx->meta_words;
   p.n_gbuf = ctx->n_gbuf;
   p.powers = ctx->use_powers ? ctx->d_powers.as<float>() : nullptr;
   p.power_floats = ctx->power_floats;
   p.off_acc = ctx->off_acc;
   p.off_gtab = ctx->off_gtab;
   p.off_stg = ctx->off_stg;
-  p.off_cnt = ctx->off_cnt;
-  p.off_off = ctx->off_off;
-  p.off_pair = ctx->off_pair;
-  p.off_ent = ctx->off_ent;
-  p.off_wsum = ctx->off_wsum;
+  p.off_q = ctx->off_q;
+  p.off_meta = ctx->off_meta;
   p.off_stages = ctx->off_stages;
-  p.fin_off = ctx->d_fin_off.as<uint32_t>();
+  p.fin_lists = ctx->d_fin_lists.as<FinList>();
   p.fin_visits = ctx->d_fin_visits.as<uint32_t>();
-  p.fin_first = ctx->fin_ranges ? ctx->d_fin_first.as<uint32_t>() : nullptr;
   p.n_groups = ctx->n_groups;
   p.cb_group = ctx->d_cb_group.as<uint32_t>();
-  p.group_cb = ctx->d_group_cb.as<uint32_t>();
+  p.n_chunks = ctx->n_chunks;
+  p.chunks = ctx->d_chunks.as<uint2>();
+  p.group_chunk = ctx->d_group_chunk.as<uint32_t>();
   p.mags_stride = ctx->mags_stride;
-  p.dir_of_sub = ctx->d_dir_of_sub.as<uint32_t>();
   p.cb_flag = ctx->d_cb_flag.as<uint32_t>();
   p.cb_avg = ctx->d_cb_avg.as<double>();
   p.cb_newflag = ctx->d_cb_done.as<uint32_t>();
@@ -5035,6 +5445,8 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.block_cnt = ctx->d_block_cnt.as<uint32_t>();
   p.counters = ctx->d_counters.as<uint32_t>();
   p.next_out = ctx->d_next.as<double2>();
+  p.n_iters = 1;
+  p.out_stride = 0;
   p.host_mode = host_mode ? 1 : 0;
   p.fin_mode = kFinFused;
   p.settings = ctx->d_settings.as<DevSettings>();
@@ -5072,11 +5484,11 @@ int LaunchPowers(ddsolve_ctx* ctx, bool force) {
   const uint32_t blocks = ctx->n_power_tiles * ctx->n_dir;
   if (blocks) {
     if (ctx->n_corr == 2)
-      power_kernel<2><<<blocks, kPipeRuns, 0, ctx->stream>>>(
+      power_kernel<2><<<blocks, uint32_t(ctx->pipe_entry->warps) * 32 / ctx->pipe_ng, 0, ctx->stream>>>(
           ctx->d_slabs.as<SlabDesc>(), ctx->d_power_tiles.as<PowerTile>(), ctx->n_dir,
           ctx->power_floats, ctx->d_powers.as<float>());
     else
-      power_kernel<4><<<blocks, kPipeRuns, 0, ctx->stream>>>(
+      power_kernel<4><<<blocks, uint32_t(ctx->pipe_entry->warps) * 32 / ctx->pipe_ng, 0, ctx->stream>>>(
           ctx->d_slabs.as<SlabDesc>(), ctx->d_power_tiles.as<PowerTile>(), ctx->n_dir,
           ctx->power_floats, ctx->d_powers.as<float>());
     DDS_CHECK_CUDA(ctx, cudaGetLastError());
@@ -5261,8 +5673,11 @@ int LaunchFullJones(ddsolve_ctx* ctx, bool host_mode, bool use_handle, bool with
   return DDSOLVE_OK;
 }
 
+// `n_passes` (pipe_kernel, without constraints): passes of the one launch --
+// a solve's iterations until it stops, or in host mode a chain of
+// next-solutions passes into consecutive slots of `out_stride` values.
 int LaunchIteration(ddsolve_ctx* ctx, bool host_mode, bool use_handle,
-                    bool with_make_finite) {
+                    bool with_make_finite, uint32_t n_passes = 1, size_t out_stride = 0) {
   if (ctx->n_pol == 4) return LaunchFullJones(ctx, host_mode, use_handle, with_make_finite);
   const bool constrained = !host_mode && !ctx->constraints.empty();
   if (ctx->use_pipe) {
@@ -5270,10 +5685,12 @@ int LaunchIteration(ddsolve_ctx* ctx, bool host_mode, bool use_handle,
     // resident (the grid is #SM x occupancy).
     PipeParams pp = MakePipeParams(ctx, host_mode, use_handle);
     if (constrained) pp.fin_mode = kFinStepOnly;
+    pp.n_iters = constrained ? 1u : n_passes;
+    pp.out_stride = out_stride;
     void* args[] = {&pp};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctx->n_ctas);
-    cfg.blockDim = dim3(kPipeThreads);
+    cfg.blockDim = dim3(uint32_t(ctx->pipe_entry->warps) * 32 + 32);
     cfg.dynamicSmemBytes = ctx->pipe_smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
@@ -5290,9 +5707,9 @@ int LaunchIteration(ddsolve_ctx* ctx, bool host_mode, bool use_handle,
     ap.fin_mode = kFinAssignOnly;
     ap.next_out = cons;
     if (ctx->n_pol == 2)
-      assign_kernel<2><<<ctx->n_ctas, kPipeRuns, 0, ctx->stream>>>(ap);
+      assign_kernel<2><<<ctx->n_ctas, kWarps * 32, 0, ctx->stream>>>(ap);
     else
-      assign_kernel<1><<<ctx->n_ctas, kPipeRuns, 0, ctx->stream>>>(ap);
+      assign_kernel<1><<<ctx->n_ctas, kWarps * 32, 0, ctx->stream>>>(ap);
     DDS_CHECK_CUDA(ctx, cudaGetLastError());
     return DDSOLVE_OK;
   }
@@ -5344,7 +5761,7 @@ int CheckDeviceError(ddsolve_ctx* ctx, bool staged = false) {
     DDS_CHECK_CUDA(ctx, cudaMemcpy(c, ctx->d_counters.ptr, 8, cudaMemcpyDeviceToHost));
   }
   if (c[1] != 0) {
-    cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream);
+    cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     return ctx->Fail(DDSOLVE_E_TIMEOUT,
                      "a bounded device wait of pipe_kernel timed out; results are invalid");
@@ -5468,6 +5885,7 @@ int ddsolve_create(const ddsolve_dims* dims, int device, ddsolve_ctx** out) {
   std::unique_ptr<ddsolve_ctx> ctx(new ddsolve_ctx());
   ctx->device = device;
   ctx->n_sm = prop.multiProcessorCount;
+  ctx->max_smem = prop.sharedMemPerBlockOptin;
   ctx->n_ant = dims->n_antennas;
   ctx->n_dir = dims->n_directions;
   ctx->n_cb = dims->n_channel_blocks;
@@ -6120,7 +6538,7 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
                                         ctx->stream));
     DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_done.ptr, 0, size_t(ctx->n_cb) * 4,
                                         ctx->stream));
-    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
     if ((rc = LaunchMakeFinite(ctx, false)) != DDSOLVE_OK) return rc;
     if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
     // The model powers are part of solving the interval: a solve recomputes
@@ -6131,7 +6549,9 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
   }
   // DDSOLVE_NO_GRAPH: host-driven launches, one per kernel (for profilers
   // that do not see kernels inside conditional graph nodes).
-  if (!ctx->graph_ok && !std::getenv("DDSOLVE_NO_GRAPH")) {
+  // pipe_kernel without constraints runs the loop itself.
+  const bool in_kernel = ctx->use_pipe && ctx->constraints.empty();
+  if (!in_kernel && !ctx->graph_ok && !std::getenv("DDSOLVE_NO_GRAPH")) {
     rc = BuildGraph(ctx);
     if (rc != DDSOLVE_OK) {
       // Conditional graphs unavailable: fall back to host-driven launches.
@@ -6139,21 +6559,29 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
       cudaGetLastError();
     }
   }
-  LoopState ls{};
   std::vector<LoopState> states(n_groups);
   const size_t n_mags = std::max(std::max(ctx->settings.max_iterations,
                                           ctx->settings.min_iterations), 1u);
   DDS_CHECK_CUDA(ctx, ctx->ReserveStage(n_mags));
   bool staged = false;
-  if (ctx->graph_ok && n_groups == 1) {
-    DDS_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
-    DDS_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_stage->ls, ctx->d_state.ptr, sizeof(ls),
+  uint32_t solve_launches = 0;
+  if (in_kernel)
+    for (size_t left = n_mags; left > 0;) {
+      const uint32_t n = uint32_t(std::min<size_t>(left, kItersPerLaunch));
+      if ((rc = LaunchIteration(ctx, false, false, false, n)) != DDSOLVE_OK) return rc;
+      left -= n;
+      ++solve_launches;
+    }
+  if ((in_kernel || ctx->graph_ok) && n_groups == 1) {
+    if (!in_kernel) DDS_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
+    DDS_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_stage->ls, ctx->d_state.ptr, sizeof(LoopState),
                                         cudaMemcpyDeviceToHost, ctx->stream));
     if (step_magnitudes)
       DDS_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage->mags, ctx->d_mags.ptr, n_mags * 8,
                                           cudaMemcpyDeviceToHost, ctx->stream));
     if ((rc = StageCounters(ctx)) != DDSOLVE_OK) return rc;
     staged = true;
+  } else if (in_kernel) {
   } else if (ctx->graph_ok) {
     DDS_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
   } else {
@@ -6193,16 +6621,18 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
                                      n * 8, cudaMemcpyDeviceToHost));
     }
   }
-  // pipe path: make_finite + build_tables (+ power_kernel) + one pipe_kernel
-  // per iteration; else three kernels per iteration (full-Jones: make_finite,
-  // the pass launches and the finalisation); with device constraints also
-  // their kernels and the assignment pass, every iteration
+  // pipe path: make_finite + build_tables (+ power_kernel) + the pipe_kernel
+  // launches (one per kItersPerLaunch iterations of the cap; with device
+  // constraints one per iteration, and the constraints' kernels and the
+  // assignment pass); else three kernels per iteration (full-Jones:
+  // make_finite, the pass launches and the finalisation)
   const uint64_t per_it_cons =
       ctx->constraints.empty() ? 0u : uint64_t(ConstraintLaunches(ctx)) + 1u;
   const uint64_t per_it = ctx->n_pol == 4 ? 2u + FjPassLaunches(ctx) : 3u;
-  ctx->last_launches = ctx->use_pipe
-                           ? uint64_t(max_it) * (1 + per_it_cons) + 2 + (solve_powers ? 1 : 0)
-                           : uint64_t(max_it) * (per_it + per_it_cons);
+  ctx->last_launches =
+      ctx->use_pipe ? (in_kernel ? solve_launches : uint64_t(max_it) * (1 + per_it_cons)) + 2 +
+                          (solve_powers ? 1 : 0)
+                    : uint64_t(max_it) * (per_it + per_it_cons);
   // the model powers are fresh for one solve only (see LaunchPowers)
   ctx->powers_dirty = true;
   if ((rc = CheckDeviceError(ctx, staged)) != DDSOLVE_OK) return rc;
@@ -6399,7 +6829,7 @@ int ddsolve_perform_iteration(ddsolve_ctx* ctx, const double* solutions,
                                         ctx->stream));
     DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_done.ptr, 0, size_t(ctx->n_cb) * 4,
                                         ctx->stream));
-    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
     if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
     powers_launched = ctx->use_powers && ctx->powers_dirty;
     if ((rc = LaunchPowers(ctx, false)) != DDSOLVE_OK) return rc;
@@ -6463,24 +6893,28 @@ int ddsolve_perform_iterations(ddsolve_ctx* ctx, const double* start, uint32_t n
   if (ctx->use_pipe) {
     // Once per call (every pipe_kernel launch leaves its counters at zero;
     // next-solutions passes use none of the solve's non-finite flags).
-    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
   }
   if (dev_in) ctx->d_sol.ptr = const_cast<double*>(start);
-  for (uint32_t k = 0; k < n_passes; ++k) {
+  if (ctx->use_pipe) {  // the chain runs in the kernel, kItersPerLaunch passes per launch
+    if (ctx->use_powers && ctx->powers_dirty) ++launches;
+    if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
+    if ((rc = LaunchPowers(ctx, false)) != DDSOLVE_OK) return rc;
+    ++launches;
+    for (uint32_t k = 0; k < n_passes; k += kItersPerLaunch) {
+      // later launches use the gain tables the one before left
+      if (k > 0) ctx->d_sol.ptr = chain + bytes * (k - 1);
+      ctx->d_next.ptr = chain + bytes * k;
+      if ((rc = LaunchIteration(ctx, true, false, false, std::min(n_passes - k, kItersPerLaunch),
+                                n_sol)) != DDSOLVE_OK)
+        return rc;
+      ++launches;
+    }
+  }
+  for (uint32_t k = 0; k < n_passes && !ctx->use_pipe; ++k) {
     if (k > 0) ctx->d_sol.ptr = chain + bytes * (k - 1);
     ctx->d_next.ptr = chain + bytes * k;
-    if (ctx->use_pipe) {
-      // pass k > 0 uses the gain tables that pass k - 1 wrote from its output
-      if (k == 0) {
-        if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
-        if (ctx->use_powers && ctx->powers_dirty) ++launches;
-        if ((rc = LaunchPowers(ctx, false)) != DDSOLVE_OK) return rc;
-        ++launches;
-      }
-      ++launches;
-    } else {
-      launches += 2;
-    }
+    launches += 2;
     if ((rc = LaunchIteration(ctx, true, false, false)) != DDSOLVE_OK) return rc;
   }
   if (!in_place_out)
@@ -6597,15 +7031,19 @@ int TimeIteration(ddsolve_ctx* ctx, uint32_t n, float* ms_out) {
   if (ctx->use_pipe) {
     DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_cb_flag.ptr, 0, size_t(ctx->n_cb) * 4,
                                         ctx->stream));
-    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, 16, ctx->stream));
+    DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
     if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
   }
   DDS_CHECK_CUDA(ctx, cudaEventRecord(c, ctx->stream));
   if ((rc = LaunchPowers(ctx, true)) != DDSOLVE_OK) return rc;
   if ((rc = LaunchIteration(ctx, true, false, false)) != DDSOLVE_OK) return rc;  // warm-up
   DDS_CHECK_CUDA(ctx, cudaEventRecord(a, ctx->stream));
-  for (uint32_t i = 0; i < n; ++i)
-    if ((rc = LaunchIteration(ctx, true, false, false)) != DDSOLVE_OK) return rc;
+  // as a solve runs them: pipe_kernel's passes in one launch
+  const uint32_t per_launch = ctx->use_pipe ? std::min(n, kItersPerLaunch) : 1u;
+  for (uint32_t i = 0; i < n; i += per_launch)
+    if ((rc = LaunchIteration(ctx, true, false, false, std::min(n - i, per_launch))) !=
+        DDSOLVE_OK)
+      return rc;
   DDS_CHECK_CUDA(ctx, cudaEventRecord(b, ctx->stream));
   DDS_CHECK_CUDA(ctx, cudaEventSynchronize(b));
   float ms = 0.f, first = 0.f;
@@ -6673,8 +7111,7 @@ int ddsolve_autotune(ddsolve_ctx* ctx, uint32_t launches, ddsolve_tuning* chosen
   }
   // candidates: pipe_kernel plan variants, then stream_kernel lane groups
   std::vector<ddsolve_tuning> cands;
-  const bool pipe_ok = (ctx->n_corr == 2 || ctx->n_corr == 4) &&
-                       FindPipeKernel(int(ctx->n_corr), int(ctx->n_pol), int(ctx->n_dir));
+  const bool pipe_ok = (ctx->n_corr == 2 || ctx->n_corr == 4) && FindPipeKernel(ctx);
   if (pipe_ok)
     for (int32_t powers : {0, 1})
       for (uint32_t gbuf : {1u, 2u})
