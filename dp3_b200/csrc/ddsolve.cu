@@ -2065,7 +2065,7 @@ __device__ __forceinline__ bool FinalizeDistributed(const PipeParams& p, uint32_
   // The items, warp by warp over the CTAs; a lane reads its slots of an item
   // kR at a time and adds them in slot order, and the lanes of the item then
   // add up theirs.
-  auto merge = [&](uint32_t item, uint32_t part) {
+  auto merge = [&](uint32_t item, const Item& x, uint32_t part) {
     const bool range = (x.list.y & kFinRange) != 0;
     // no partial slots to merge after the constraints
     const uint32_t count = p.fin_mode == kFinAssignOnly ? 0u : x.list.y & ~kFinRange;
@@ -2074,7 +2074,8 @@ __device__ __forceinline__ bool FinalizeDistributed(const PipeParams& p, uint32_
     const float* den =
         p.partials + size_t(x.ant) * p.acc_stride + AccDenOffset(NPOL, p.n_dir, x.list.z, 0);
     NeumaierSum nr[NPOL], ni[NPOL], dn[NPOL];
-    constexpr uint32_t kR = 4;  // slots per round (8 at once spill the row loop)
+    // slots per round (8 at once spill the row loop of kWarps warps)
+    constexpr uint32_t kR = W == kWideWarps ? 6 : 4;
     for (uint32_t k = part * kR; k < count; k += kR << share) {
       float v[kR][NPOL * 3];
 #pragma unroll
@@ -2111,9 +2112,9 @@ __device__ __forceinline__ bool FinalizeDistributed(const PipeParams& p, uint32_
   };
   if (single) {
     for (uint32_t i = item_first; (i >> share) < n_items; i += item_step) {
-      const uint32_t item = i >> share;
-      if (i != item_first) fetch(item, x);
-      merge(item, i & ((1u << share) - 1u));
+      const Item now = x;
+      if (((i + item_step) >> share) < n_items) fetch((i + item_step) >> share, x);
+      merge(i >> share, now, i & ((1u << share) - 1u));
     }
     FenceProxyAsync();  // the gain tables, before the next pass's bulk copies
     BlockNorm<W>(ctid, nsum, ncnt, bad, s_sum, s_cnt);
@@ -2135,7 +2136,7 @@ __device__ __forceinline__ bool FinalizeDistributed(const PipeParams& p, uint32_
     if (uint32_t(ctid & 31) < chunk.y >> 24) {
       const uint32_t item = chunk.x + uint32_t(ctid & 31);
       fetch(item, x);
-      merge(item, 0);
+      merge(item, x, 0);
     }
     __syncwarp();
 #pragma unroll
@@ -2354,16 +2355,17 @@ __device__ __forceinline__ void GatherEntries(const uint32_t (&en)[kGather], uin
     }
     if constexpr (NPOL == 1) {
       // one gain for every correlation: their sums are staged
-      const float4* const v_at = SharedPtr<const float4>(stg_at + j * (RUNS * 16));
+      const float2* const v_at = SharedPtr<const float2>(stg_at + j * (RUNS * 8));
+      const float* const z_at = SharedPtr<const float>(q_at + j * (RUNS * 4));
 #pragma unroll
       for (uint32_t u = 0; u < kGather; ++u) {
         if (u >= n) break;
         const float2 gc = *SharedPtr<const float2>(gains[u] + j * 8);
-        const float4 v = v_at[run[u]];
+        const float2 v = v_at[run[u]];
         const float vy = __uint_as_float(__float_as_uint(v.y) ^ ((en[u] << 16) & 0x80000000u));
         num[0].x = fmaf(gc.x, v.x, fmaf(-gc.y, vy, num[0].x));
         num[0].y = fmaf(gc.x, vy, fmaf(gc.y, v.x, num[0].y));
-        den[0] = fmaf(cnorm(gc), v.z, den[0]);
+        den[0] = fmaf(cnorm(gc), z_at[run[u]], den[0]);
       }
     } else {
       const uint32_t p_at = stg_at + j * (RUNS * NCORR * 8);
@@ -2415,13 +2417,12 @@ __device__ __forceinline__ void GatherEntries(const uint32_t (&en)[kGather], uin
 // The second half of a tile's reduction: the antennas' sums over the staged
 // directions d0 .. d0 + n_staged - 1, P at stg[j][run][corr] and the model
 // powers at q[j][run][corr] (0: none in this fragment); for one polarization
-// their sums over the correlations at stg[j][run] as P, Q, 0. Thread (i, j0) adds up
+// their sums over the correlations, P at stg[j][run] and Q at q[j][run]. Thread (i, j0) adds up
 // antenna i (and i + (W * 32), ...) for the staged directions j0, j0 +
 // step, ..., over the antenna's entries in their order, kGather entries per
 // update of an accumulator: few barriers and read-modify-write chains,
 // whatever the order of the runs. Consecutive threads take consecutive
-// antennas, mostly of consecutive runs: distinct shared-memory banks. Out of
-// line: its registers would spill the row loop.
+// antennas, mostly of consecutive runs: distinct shared-memory banks.
 template <int W, int NCORR, int NPOL, int RUNS>
 __device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, uint32_t stg_at,
                                         uint32_t q_at, uint32_t acc_at, uint32_t ctid,
@@ -2456,12 +2457,15 @@ __device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, u
 // lane g of a run owns directions g, g + NG, ... (DPL of them); the residual
 // is the sum over the run's lanes (warp shuffles). NG = 1: one run per lane,
 // exactly DPL directions.
-// Bound: HBM, as long as the rows' arithmetic hides under their copies. With
-// 7 consumer warps of 255 registers (two per scheduler) a row of a
-// 62-station, 10-direction interval took 0.55 us of waiting and dependent
-// arithmetic against 0.9 us of copy, and a tile's reduction 6.8 us: at most
-// DPL = 5 directions a lane keep a thread within 128 registers, so that 15
-// warps cover each other's latencies.
+// Bound: HBM (6.2 of 6.5 TB/s measured for a copy) while rows stream, and
+// latency in the end of a pass. 11 consumer warps of at most DPL = 5
+// directions a lane, in 168 registers without spills, cover each other's
+// latencies: a 31 KB row (62 stations, 10 directions) takes 0.6 us, the time
+// of its copy, a tile's reduction 2.0 us; 7 warps of up to 10 directions a lane
+// took 6.8 us for the reduction. One launch runs many passes, and the ring
+// fills with the next pass's rows while the grid finalises: 24 channel blocks
+// of 80 rows (240 channels, 8 times) 125 -> 103 us a pass, 12 blocks of 20 rows
+// 43 -> 19 us.
 // SUMQ: the model powers are summed in the row loop (else precomputed).
 constexpr int kPairValues = 6;  // model values per lane up to which two rows fit its registers
 // Of a lane's directions, staged at a time: all, or three with more than
@@ -2922,7 +2926,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
             const uint32_t j = g + (k - k0) * NG;  // staged direction k0 * NG + j
             if (k < DPL - 1 || last_mine) {
 if constexpr (NPOL == 1) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                float3 v = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < NCORR; ++c) {
                   v.x += P[k][c].x;
@@ -2935,7 +2939,8 @@ if constexpr (NPOL == 1) {
 #pragma unroll
                   for (int c = 0; c < NCORR; ++c) v.z += q[c];
                 }
-                stg[j * RUNS + run] = v;
+                reinterpret_cast<float2*>(stg)[j * RUNS + run] = make_float2(v.x, v.y);
+                reinterpret_cast<float*>(stg_q)[j * RUNS + run] = v.z;
               } else {
 #pragma unroll
                 for (int h = 0; h < NCORR / 2; ++h)
@@ -2954,7 +2959,9 @@ if constexpr (NPOL == 1) {
         ConsumerBarrier<W>();
         const uint32_t d0 = k0 * NG;
         const uint32_t n_staged = min(uint32_t(StageDirs(W) * NG), n_dir - d0);
-        const uint32_t q_from = q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4 : q_src;
+        const uint32_t q_from = NPOL == 1          ? SmemAddr(stg_q)
+                                : q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4
+                                                 : q_src;
         GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), SmemAddr(stg), q_from,
                                       SmemAddr(acc), ctid, n_dir, d0, n_staged, p.acc_stride,
                                       p.gain_stride);
@@ -4238,9 +4245,12 @@ PipeLayout MakePipeLayout(const ddsolve_ctx* ctx, uint32_t ng, uint32_t warps, u
   off += n_gbuf * table_f2 * 8;
   l.off_stg = uint32_t(off);
   const size_t staged = std::min<size_t>(n_dir, StageDirs(int(warps)) * ng);
-  off += staged * runs * (ctx->n_pol == 1 ? 16 : n_corr * 8);
+  off += staged * runs * (ctx->n_pol == 1 ? 1 : n_corr) * 8;
   l.off_q = uint32_t(off);
-  if (stage_q && ctx->n_pol != 1) off += staged * n_corr * runs * 4;
+  if (ctx->n_pol == 1)
+    off += staged * runs * 4;
+  else if (stage_q)
+    off += staged * n_corr * runs * 4;
   l.off_meta = uint32_t(off = align(off, 16));
   l.meta_words = MetaWords(uint32_t(runs), ctx->n_ant);
   off += 2 * size_t(l.meta_words) * 4;
@@ -4258,8 +4268,10 @@ PipeLayout MakePipeLayout(const ddsolve_ctx* ctx, uint32_t ng, uint32_t warps, u
 // when no variant fits. It depends on the dimensions only, so that every
 // upload packs the tiles that the plan will use. Two correlations with more
 // than 20 directions take four lanes of up to 12 directions each in the wide
-// variant: eight lanes of 5 with kWarps measured 443 us a pass against 360 for
+// variant: eight lanes of 5 with kWarps measured 443 us a pass against 329 for
 // 40 directions on 62 stations (twelve shuffles a row for five directions).
+// Fewer than three stages cost more than the shuffles of more lanes; from three
+// on the fewer lanes win (512 stations, 5 directions: 263 us against 320).
 const KernelEntry* FindPipeKernel(const ddsolve_ctx* ctx) {
   const KernelEntry* best = nullptr;
   uint32_t best_stages = 0;
@@ -4798,10 +4810,10 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   // ---- fragments: rows balanced over the CTAs ----
   // A row weighs its bytes; every fragment, whole tile or part of one, adds
   // its reduction: 2.3 us against 0.7 us for a 31 KB row (62 stations, 10
-  // directions), 3.5 us where the directions are staged in two parts. The
+  // directions), 4.5 us against 0.6 us for a 37 KB row in the wide variant. The
   // least bound under which filling the CTAs in order covers all rows is
   // found by bisection.
-  const double reduce_bytes = ctx->pipe_entry->warps == kWideWarps ? 160e3 : 100e3;
+  const double reduce_bytes = ctx->pipe_entry->warps == kWideWarps ? 340e3 : 100e3;
   auto row_cost = [&](const Tile& t) { return double(t.n) * (1 + n_dir) * ctx->elem_bytes + 1e3; };
   auto frag_cost = [&](const Tile&) { return reduce_bytes; };
   uint64_t total_rows = 0;
@@ -4893,14 +4905,19 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
 
   // ---- shared-memory layout ----
   // Two gain-table buffers (the next visit's table loads while the current
-  // one is in use) unless that leaves fewer than three stages, or as asked for
-  // where two stages still fit.
+  // one is in use) unless that leaves fewer than four stages and one leaves
+  // more, or as asked for where two stages still fit: 512 stations, 5
+  // directions, one polarization, 3 against 4 stages: 277 -> 263 us
+  // a pass.
   const uint32_t warps = uint32_t(ctx->pipe_entry->warps);
   uint32_t n_gbuf = ctx->tune_gbuf == 1 ? 1u : 2u;
   PipeLayout lay = MakePipeLayout(ctx, ctx->pipe_ng, warps, n_gbuf, !use_powers);
-  if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 3u)) {
-    n_gbuf = 1;
-    lay = MakePipeLayout(ctx, ctx->pipe_ng, warps, n_gbuf, !use_powers);
+  if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 4u)) {
+    const PipeLayout one = MakePipeLayout(ctx, ctx->pipe_ng, warps, 1, !use_powers);
+    if (one.stages > lay.stages) {
+      n_gbuf = 1;
+      lay = one;
+    }
   }
   uint32_t stages = lay.stages;
   if (ctx->tune_stages >= 2) stages = std::min(stages, ctx->tune_stages);
@@ -6581,10 +6598,9 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
                                           cudaMemcpyDeviceToHost, ctx->stream));
     if ((rc = StageCounters(ctx)) != DDSOLVE_OK) return rc;
     staged = true;
-  } else if (in_kernel) {
-  } else if (ctx->graph_ok) {
+  } else if (ctx->graph_ok && !in_kernel) {
     DDS_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
-  } else {
+  } else if (!in_kernel) {
     const uint32_t cap = std::max(std::max(ctx->settings.max_iterations,
                                            ctx->settings.min_iterations), 1u);
     for (uint32_t it = 0; it < cap; ++it) {

@@ -489,7 +489,8 @@ DDSOLVE_API int ddsolve_perform_iteration_noalloc(
     const uint32_t* antenna1, const uint32_t* antenna2,
     const double* solutions, double* next_solutions, void* stream);
 
-/* Number of kernel launches issued by the last ddsolve_solve call. */
+/* Number of kernel launches issued by the last ddsolve_solve call (an
+ * unconstrained solve on the pipelined path runs up to 64 iterations in one). */
 DDSOLVE_API uint64_t ddsolve_last_launch_count(const ddsolve_ctx* ctx);
 
 #ifdef __cplusplus
