@@ -1455,11 +1455,12 @@ struct PipeShared {
   uint64_t gfull[2], gfree[2];  // gain table buffer loaded / released
   uint64_t mfree[2];            // antenna buffer released
   // Thread 0 polls the grid's counters for its CTA and passes the news on to
-  // the consumers: every partial slot of the pass is written; the pass is
-  // finished (with `stop`: so is the launch). One phase per pass each. The
-  // producer, which no barrier keeps within a phase of the consumers, reads
-  // the number of finished passes instead.
-  uint64_t flushed, ready;
+  // the consumers: every partial slot of the pass is written; every CTA has
+  // finalised it (in the CTA of the control step only); the pass is finished
+  // (with `stop`: so is the launch). One phase per pass each. The producer,
+  // which no barrier keeps within a phase of the consumers, reads the number
+  // of finished passes instead.
+  uint64_t flushed, finalised, ready;
   double sum[16];  // the warps' norm partials
   uint32_t cnt[32];
   uint32_t flag[2];
@@ -2307,9 +2308,12 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
     sh.bad_seen = uint32_t(count >> 32);
     if (!done) sh.stop = 1u;
     sh.flag[1] = all_bad ? 1u : 0u;
+    if (control && is_control) MbarArrive(&sh.finalised);
   }
   if (control && is_control) {
-    ConsumerBarrier<W>();
+    // (every warp waits for the news itself: no named barrier right after
+    // thread 0's polling, see ConsumerBarrier)
+    PipeWait(&sh.finalised, it & 1u, &sh.err, &p.counters[kCntError]);
     const uint32_t v = ControlPass<W, NPOL>(p, ctid, sh.flag[1] != 0, sh.sum, sh.cnt, sh.flag);
     if (ctid == 0) {
       p.counters[kCntVerdict] = v;
@@ -2538,6 +2542,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
       MbarInit(&mfree[b], W);
     }
     MbarInit(&sh.flushed, 1);
+    MbarInit(&sh.finalised, 1);
     MbarInit(&sh.ready, 1);
     sh.err = 0;
     sh.stop = 0;

@@ -1,0 +1,64 @@
+"""The control step of the pipelined solve: the CTA that runs it replaces the
+non-finite solutions of a pass and decides on every interval of a batch, with
+all of its warps, once every CTA has finalised the pass.
+
+Tolerance: 1e-4, the parity contract of a solve (after phase referencing; the
+replaced solutions, means of amplitudes of solved ones, as they are).
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle_ffi as of
+from tests import helpers as H
+
+RTOL_SOLVE = 1e-4
+
+
+def _flag_antenna(prob, antenna, blocks):
+    """Zeroes an antenna's visibilities in some channel blocks: its denominator
+    is zero there and its solutions are replaced after every pass."""
+    for cb in blocks:
+        ap = prob["antenna_pairs"][cb]
+        bad = (ap[:, 0] == antenna) | (ap[:, 1] == antenna)
+        prob["data"][cb][bad] = 0
+        prob["model"][cb][:, bad] = 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_dir,n_st,n_intervals", [(2, 9, 1), (2, 9, 5), (21, 30, 3)])
+def test_non_finite_blocks_of_every_interval(built, n_dir, n_st, n_intervals):
+    """One interval and batches, each interval with an antenna of its own
+    flagged in its last channel block (11 and 7 consumer warps)."""
+    from dp3_b200 import ddsolve
+    n_it, n_cb = 12, 3
+    probs, refs, its = [], [], []
+    for g in range(n_intervals):
+        obs = H.small_observation(n_stations=n_st, n_directions=n_dir, n_channels=6, n_cb=n_cb,
+                                  n_times=2, seed=40 + g, n_sources=2)
+        prob = H.problem_from_observation(obs)
+        _flag_antenna(prob, 1 + g, [n_cb - 1])
+        ref = H.unit_solutions(prob)
+        r, _ = of.solve(prob, ref, of.settings(max_iterations=n_it, accuracy=1e-30,
+                                               detect_stalling=False), precision=64, n_threads=2)
+        probs.append(prob)
+        refs.append(ref)
+        its.append(r.iterations)
+    st = ddsolve.default_settings()
+    st.max_iterations, st.accuracy, st.detect_stalling = n_it, 1e-30, 0
+    ctx = ddsolve.Context(n_st, [1] * n_dir, n_intervals * n_cb, 2, 2)
+    ctx.set_settings(st)
+    if n_intervals > 1:
+        ctx.set_intervals([g * n_cb for g in range(n_intervals + 1)])
+    for g, prob in enumerate(probs):
+        for cb in range(n_cb):
+            ctx.set_channel_block(g * n_cb + cb, prob["data"][cb], prob["model"][cb],
+                                  prob["antenna_pairs"][cb], prob["solution_map"][cb])
+    sol = np.ones((n_intervals * n_cb,) + refs[0].shape[1:], np.complex128)
+    res = ctx.solve_batch(sol) if n_intervals > 1 else [ctx.solve(sol)]
+    ctx.close()
+    for g, ref in enumerate(refs):
+        got = sol[g * n_cb:(g + 1) * n_cb]
+        assert res[g].iterations == its[g]
+        np.testing.assert_allclose(got[-1, 1 + g], ref[-1, 1 + g], rtol=RTOL_SOLVE)
+        ok = np.arange(n_st) != 1 + g
+        assert H.max_rel_diff(got[:, ok], ref[:, ok]) < RTOL_SOLVE
