@@ -1360,7 +1360,7 @@ constexpr int kWarps = 11, kWideWarps = 7;
 // and sums fit 255.
 constexpr uint32_t kPipeDirs2 = 5, kPipeDirs4 = 3, kPipeDirsWide = 12;
 constexpr int kPipeMaxStages = 8;
-constexpr uint64_t kWaitBudgetNs = 4000000000ull;
+constexpr uint64_t kWaitNs = 4000000000ull;  // limit of a device wait
 
 // Device counters of pipe_kernel, each polled word on a cache line of its
 // own. The error flag (a bounded wait ran out). Arrivals of CTAs whose partial
@@ -1447,6 +1447,10 @@ struct PipeParams {
   uint32_t n_chunks;
   const uint2* chunks;
   const uint32_t* group_chunk;
+  // The limit of every device wait, and arrivals that the grid barrier expects
+  // beyond those of its CTAs (none but in ddsolve_check_wait_limit).
+  uint64_t wait_ns;
+  uint32_t arrive_extra;
 };
 
 // The head of pipe_kernel's shared memory.
@@ -1464,6 +1468,7 @@ struct PipeShared {
   double sum[16];  // the warps' norm partials
   uint32_t cnt[32];
   uint32_t flag[2];
+  uint32_t skip;  // the launch does nothing
   volatile uint32_t stop, passes;
   volatile int err;
   // thread 0: the counters before the launch, non-finite arrivals so far, the
@@ -1473,7 +1478,8 @@ struct PipeShared {
 };
 
 // A fragment of an interval that has stopped: skipped by the producer and the
-// consumers alike (the loop states do not change during a launch).
+// consumers alike: with several intervals no pass begins before the control
+// step of the one before it, and none runs while a CTA is in its rows.
 __device__ __forceinline__ bool FragFrozen(const PipeParams& p, uint32_t slab) {
   if (p.n_groups <= 1 || p.host_mode) return false;
   const uint32_t g = p.cb_group[p.slabs[slab].cb];
@@ -1562,27 +1568,44 @@ __device__ __forceinline__ void ConsumerBarrier() {
 
 // Bounded wait on an mbarrier phase. Returns false on timeout (or when the CTA
 // is already in error), after recording the error.
-__device__ __forceinline__ bool PipeWaitSlow(uint64_t* bar, uint32_t parity, volatile int* s_err,
-                                             uint32_t* g_err) {
+__device__ __forceinline__ bool PipeWaitSlow(uint64_t* bar, uint32_t parity, PipeShared& sh) {
   uint64_t t0 = 0;
   for (uint32_t n = 1;; ++n) {
     if (MbarTryWait(bar, parity)) return true;
     if ((n & 15u) == 0) {  // (reading the timer is slow)
-      if (*s_err) return false;
+      if (sh.err) return false;
       const uint64_t t = GlobalTimerNs();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kWaitBudgetNs) {
-        *s_err = 1;
-        atomicExch(g_err, 1u);
+      if (t - t0 > sh.params.wait_ns) {
+        sh.err = 1;
+        atomicExch(&sh.params.counters[kCntError], 1u);
         return false;
       }
     }
   }
 }
-__device__ __forceinline__ bool PipeWait(uint64_t* bar, uint32_t parity, volatile int* s_err,
-                                         uint32_t* g_err) {
+__device__ __forceinline__ bool PipeWait(uint64_t* bar, uint32_t parity, PipeShared& sh) {
   if (MbarTryWait(bar, parity)) return true;
-  return PipeWaitSlow(bar, parity, s_err, g_err);
+  return PipeWaitSlow(bar, parity, sh);
+}
+
+// The consumers' wait for thread 0's news of the grid. What they do next
+// depends on it, and a warp that gave up by itself would miss named barriers at
+// which the others wait for good. Thread 0 always passes the news on: between
+// two of them it waits at most twice, each time within the limit, so the limit
+// here, four times that, is not reached.
+__device__ __forceinline__ void NewsWait(uint64_t* bar, uint32_t parity, PipeShared& sh) {
+  uint64_t t0 = 0;
+  for (uint32_t n = 1; !MbarTryWait(bar, parity); ++n) {
+    if ((n & 15u) != 0) continue;
+    const uint64_t t = GlobalTimerNs();
+    if (t0 == 0) t0 = t;
+    if (t - t0 > 4 * sh.params.wait_ns) {
+      sh.err = 1;
+      atomicExch(&sh.params.counters[kCntError], 1u);
+      return;
+    }
+  }
 }
 
 __device__ __forceinline__ uint64_t LoadAcquire64(const uint64_t* p) {
@@ -1593,14 +1616,14 @@ __device__ __forceinline__ uint64_t LoadAcquire64(const uint64_t* p) {
 // Thread 0's bounded wait until reached() holds; false when it ran out or an
 // error is flagged.
 template <typename Reached>
-__device__ __forceinline__ bool GridWait(uint32_t* counters, const Reached& reached) {
+__device__ __forceinline__ bool GridWait(const PipeParams& p, const Reached& reached) {
   const uint64_t t0 = GlobalTimerNs();
   for (uint32_t n = 1;; ++n) {
     if (reached()) return true;
     if ((n & 63u) == 0) {
-      if (static_cast<volatile uint32_t*>(counters)[kCntError]) return false;
-      if (GlobalTimerNs() - t0 > kWaitBudgetNs) {
-        atomicExch(&counters[kCntError], 1u);
+      if (static_cast<volatile uint32_t*>(p.counters)[kCntError]) return false;
+      if (GlobalTimerNs() - t0 > p.wait_ns) {
+        atomicExch(&p.counters[kCntError], 1u);
         return false;
       }
     }
@@ -2266,12 +2289,12 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
   bool bad;
   const bool go = FinalizeDistributed<W, NPOL>(p, it, ctid, sh.sum, sh.cnt, bad, [&]() {
     if (ctid == 0) {
-      const uint32_t target = (it + 1) * gridDim.x;
-      GridWait(p.counters,
+      const uint32_t target = (it + 1) * gridDim.x + p.arrive_extra;
+      GridWait(p,
                [&]() { return LoadAcquire(&p.counters[kCntArrive]) - sh.arrive0 >= target; });
       if (control && it > 0) {
         const bool known = GridWait(
-            p.counters, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it; });
+            p, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it; });
         uint32_t v = kVerdictStop;
         if (known) v = static_cast<volatile uint32_t*>(p.counters)[kCntVerdict];
         sh.verdict = v;
@@ -2283,7 +2306,7 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
       }
       MbarArrive(&sh.flushed);
     }
-    PipeWait(&sh.flushed, it & 1u, &sh.err, &p.counters[kCntError]);
+    NewsWait(&sh.flushed, it & 1u, sh);
     return sh.stop == 0u;
   });
   if (!go) return false;
@@ -2300,21 +2323,26 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
               1ull | (bad ? 1ull << 32 : 0ull));
     uint64_t count = 0;
     const uint32_t target = (it + 1) * gridDim.x;
-    const bool done = GridWait(p.counters, [&]() {
+    const bool done = GridWait(p, [&]() {
       count = LoadAcquire64(reinterpret_cast<const uint64_t*>(p.counters + kCntFinal));
       return uint32_t(count) - sh.final0 >= target;
     });
     all_bad = uint32_t(count >> 32) != sh.bad_seen;
     sh.bad_seen = uint32_t(count >> 32);
     if (!done) sh.stop = 1u;
-    sh.flag[1] = all_bad ? 1u : 0u;
+    sh.flag[1] = !done ? 2u : all_bad ? 1u : 0u;
     if (control && is_control) MbarArrive(&sh.finalised);
   }
   if (control && is_control) {
     // (every warp waits for the news itself: no named barrier right after
     // thread 0's polling, see ConsumerBarrier)
-    PipeWait(&sh.finalised, it & 1u, &sh.err, &p.counters[kCntError]);
-    const uint32_t v = ControlPass<W, NPOL>(p, ctid, sh.flag[1] != 0, sh.sum, sh.cnt, sh.flag);
+    NewsWait(&sh.finalised, it & 1u, sh);
+    // Where the wait ran out there is no control step: another CTA may still be
+    // in the rows of the pass, whose fragments depend on which intervals go on.
+    const uint32_t news = sh.flag[1];
+    const uint32_t v =
+        news == 2u ? kVerdictStop
+                   : ControlPass<W, NPOL>(p, ctid, news != 0u, sh.sum, sh.cnt, sh.flag);
     if (ctid == 0) {
       p.counters[kCntVerdict] = v;
       StoreRelease(&p.counters[kCntEpoch], sh.epoch0 + it + 1);
@@ -2324,7 +2352,7 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
   if (ctid == 0) {
     if (control && (it == 0 || all_bad || p.n_groups > 1 || (sh.verdict & kVerdictNear))) {
       const bool known = GridWait(
-          p.counters, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it + 1; });
+          p, [&]() { return LoadAcquire(&p.counters[kCntEpoch]) - sh.epoch0 >= it + 1; });
       uint32_t v = kVerdictStop;
       if (known) v = static_cast<volatile uint32_t*>(p.counters)[kCntVerdict];
       sh.verdict = v;
@@ -2334,7 +2362,8 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
     sh.passes = it + 1;
     MbarArrive(&sh.ready);
   }
-  return PipeWait(&sh.ready, it & 1u, &sh.err, &p.counters[kCntError]) && sh.stop == 0u;
+  NewsWait(&sh.ready, it & 1u, sh);
+  return sh.stop == 0u;
 }
 
 // What a tile's fragments need of its runs besides the visibilities, one
@@ -2498,15 +2527,6 @@ template <int NCORR, int NPOL, int DPL, int NG, bool SUMQ, int W>
 __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p) {
   static_assert(32 % NG == 0, "lanes per run must divide a warp");
   constexpr int RUNS = (W * 32) / NG;  // runs per tile
-  // A solve may be several launches (of kItersPerLaunch iterations, or the
-  // unrolled body of a constrained solve's graph): a launch after the solve
-  // has stopped does nothing.
-  if (!p.host_mode) {
-    bool all_done = true;
-    for (uint32_t g = 0; g < p.n_groups && all_done; ++g)
-      all_done = static_cast<volatile const LoopState*>(p.state)[g].done != 0;
-    if (all_done) return;
-  }
   extern __shared__ __align__(128) unsigned char smem[];
   PipeShared& sh = *reinterpret_cast<PipeShared*>(smem);
   uint64_t* full = sh.full;
@@ -2514,7 +2534,6 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
   uint64_t* gfull = sh.gfull;
   uint64_t* gfree = sh.gfree;
   uint64_t* mfree = sh.mfree;
-  volatile int* s_err = &sh.err;
   float* acc = reinterpret_cast<float*>(smem + p.off_acc);
   float2* gtab_buf = reinterpret_cast<float2*>(smem + p.off_gtab);
   float4* stg = reinterpret_cast<float4*>(smem + p.off_stg);
@@ -2548,6 +2567,17 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
     sh.stop = 0;
     sh.passes = 0;
     sh.params = p;
+    // A solve may be several launches (of kItersPerLaunch iterations, or the
+    // unrolled body of a constrained solve's graph): a launch after the solve
+    // has stopped, or after an error, does nothing. One thread looks: the
+    // error may be flagged while it does, and the warps have to agree.
+    bool skip = static_cast<volatile uint32_t*>(p.counters)[kCntError] != 0;
+    if (!p.host_mode && !skip) {
+      skip = true;
+      for (uint32_t g = 0; g < p.n_groups && skip; ++g)
+        skip = static_cast<volatile const LoopState*>(p.state)[g].done != 0;
+    }
+    sh.skip = skip ? 1u : 0u;
     // The counters before this launch. Those of finished passes and control
     // steps cannot move before this CTA has arrived at its first grid barrier;
     // other CTAs may have arrived there once each already.
@@ -2560,9 +2590,10 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
     sh.arrive0 = arrived - arrived % gridDim.x;
     sh.verdict = kVerdictNear;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (p.use_handle && blockIdx.x == 0) cudaGraphSetConditional(p.handle, 0);
+    if (!skip && p.use_handle && blockIdx.x == 0) cudaGraphSetConditional(p.handle, 0);
   }
   __syncthreads();
+  if (sh.skip) return;
 
   const uint32_t f_begin = p.cta_frag_off[blockIdx.x];
   const uint32_t f_end = p.cta_frag_off[blockIdx.x + 1];
@@ -2588,9 +2619,9 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         if (!tables_ready) {
           const uint64_t t0 = GlobalTimerNs();
           for (uint32_t n = 1; sh.passes < it; ++n) {
-            if (*s_err) return false;
-            if ((n & 63u) == 0 && GlobalTimerNs() - t0 > kWaitBudgetNs) {
-              *s_err = 1;
+            if (sh.err) return false;
+            if ((n & 63u) == 0 && GlobalTimerNs() - t0 > p.wait_ns) {
+              sh.err = 1;
               atomicExch(&p.counters[kCntError], 1u);
               return false;
             }
@@ -2603,7 +2634,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         if (pending == 0xFFFFFFFFu) return true;
         const uint32_t b = nvis % p.n_gbuf;
         const uint32_t use = nvis / p.n_gbuf;  // earlier uses of buffer b
-        if (use >= 1 && !PipeWait(&gfree[b], (use - 1) & 1u, s_err, &p.counters[kCntError]))
+        if (use >= 1 && !PipeWait(&gfree[b], (use - 1) & 1u, sh))
           return false;
         MbarArriveExpectTx(&gfull[b], table_bytes);
         BulkCopyG2S(gtab_buf + size_t(b) * p.table_f2, p.tables + size_t(pending) * p.table_f2,
@@ -2641,7 +2672,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         // still pending cannot move before it.
         auto take_stage = [&]() {
           if (pending != 0xFFFFFFFFu && row - row0 >= S && !fetch_table()) return false;
-          return row < S || PipeWait(&empty[st], ph ^ 1u, s_err, &p.counters[kCntError]);
+          return row < S || PipeWait(&empty[st], ph ^ 1u, sh);
         };
         // The antenna buffer of the fragment before the last, which (like the
         // ring) is not released before its gain table has arrived.
@@ -2649,8 +2680,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
           ok = false;
           break;
         }
-        if (nfrag >= 2 && !PipeWait(&mfree[nfrag & 1u], (nfrag / 2 - 1) & 1u, s_err,
-                                    &p.counters[kCntError])) {
+        if (nfrag >= 2 && !PipeWait(&mfree[nfrag & 1u], (nfrag / 2 - 1) & 1u, sh)) {
           ok = false;
           break;
         }
@@ -2698,11 +2728,11 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
     // Wait for the last copies, so none is in flight when the CTA ends.
     for (uint32_t k = 0; k < S && k < row; ++k) {
       const uint32_t r = row - 1 - k;
-      PipeWait(&full[r % S], (r / S) & 1u, s_err, &p.counters[kCntError]);
+      PipeWait(&full[r % S], (r / S) & 1u, sh);
     }
     for (uint32_t k = 0; k < p.n_gbuf && k < nvis; ++k) {
       const uint32_t v = nvis - 1 - k;
-      PipeWait(&gfull[v % p.n_gbuf], (v / p.n_gbuf) & 1u, s_err, &p.counters[kCntError]);
+      PipeWait(&gfull[v % p.n_gbuf], (v / p.n_gbuf) & 1u, sh);
     }
     return;
   }
@@ -2752,7 +2782,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         for (uint32_t i = ctid; i < acc_n / 4; i += (W * 32))
           z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         const uint32_t b = nvis % p.n_gbuf;
-        PipeWait(&gfull[b], (nvis / p.n_gbuf) & 1u, s_err, &p.counters[kCntError]);
+        PipeWait(&gfull[b], (nvis / p.n_gbuf) & 1u, sh);
         gtab = gtab_buf + size_t(b) * p.table_f2;
         cur_visit = f.visit;
         ++nvis;
@@ -2777,7 +2807,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
           if constexpr (SUMQ) Q[k][c] = 0.f;
         }
       const uint32_t n_rows = f.row_hi - f.row_lo;
-      PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+      PipeWait(&full[st], ph, sh);
       if (warp_busy) {  // with the first row: the run's antennas, gain products
         const uint32_t ap = active ? meta[kMetaRuns + run] : 0u;
         const uint32_t a1 = ap & 0xFFFFu, a2 = ap >> 16;
@@ -2808,7 +2838,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         uint32_t stage[NR];
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
-          PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+          PipeWait(&full[st], ph, sh);
           stage[i] = st;
           if (++st == S) {
             st = 0;
@@ -2932,7 +2962,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
       if (flags & kFragPower) {
         // the tile's precomputed model powers, in the stage after its rows
         q_stage = st;
-        PipeWait(&full[st], ph, s_err, &p.counters[kCntError]);
+        PipeWait(&full[st], ph, sh);
         if (++st == S) {
           st = 0;
           ph ^= 1u;
@@ -3994,6 +4024,8 @@ struct ddsolve_ctx {
   uint32_t off_acc = 0, off_gtab = 0, off_stg = 0, off_q = 0, off_meta = 0, off_stages = 0;
   DevBuf d_metas;
   uint32_t n_ctas = 0, n_visits = 0, fin_blocks = 0;
+  uint64_t wait_ns = kWaitNs;  // see PipeParams
+  uint32_t arrive_extra = 0;
   // precomputed model powers (pipe_kernel), refreshed after every upload
   bool use_powers = false, powers_dirty = true;
   uint32_t n_power_tiles = 0, power_floats = 0;
@@ -5478,6 +5510,8 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.n_chunks = ctx->n_chunks;
   p.chunks = ctx->d_chunks.as<uint2>();
   p.group_chunk = ctx->d_group_chunk.as<uint32_t>();
+  p.wait_ns = ctx->wait_ns;
+  p.arrive_extra = ctx->arrive_extra;
   p.mags_stride = ctx->mags_stride;
   p.cb_flag = ctx->d_cb_flag.as<uint32_t>();
   p.cb_avg = ctx->d_cb_avg.as<double>();
@@ -6698,6 +6732,24 @@ int ddsolve_solve(ddsolve_ctx* ctx, double* solutions, ddsolve_result* result,
     return ctx->Fail(DDSOLVE_E_STATE,
                      "the context holds several intervals: use ddsolve_solve_batch");
   return SolveImpl(ctx, solutions, result, step_magnitudes);
+}
+
+int ddsolve_check_wait_limit(ddsolve_ctx* ctx, uint32_t wait_ms) {
+  if (!ctx || wait_ms == 0) return DDSOLVE_E_INVALID;
+  int rc;
+  cudaSetDevice(ctx->device);
+  if (ctx->plan_dirty && (rc = BuildPlan(ctx)) != DDSOLVE_OK) return rc;
+  if (!ctx->use_pipe || !ctx->constraints.empty())
+    return ctx->Fail(DDSOLVE_E_UNSUPPORTED,
+                     "only unconstrained solves on the pipelined path wait across the grid");
+  std::vector<double> solutions(size_t(ctx->n_cb) * ctx->n_ant * ctx->n_sub * ctx->n_pol * 2, 1.0);
+  std::vector<ddsolve_result> results(ctx->n_groups);
+  ctx->wait_ns = uint64_t(wait_ms) * 1000000u;
+  ctx->arrive_extra = 1;
+  rc = SolveImpl(ctx, solutions.data(), results.data(), nullptr);
+  ctx->wait_ns = kWaitNs;
+  ctx->arrive_extra = 0;
+  return rc;
 }
 
 int ddsolve_solve_batch(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,

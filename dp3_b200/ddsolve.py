@@ -29,6 +29,7 @@ EXPORTED_SYMBOLS = (
     "ddsolve_set_interval_buffers", "ddsolve_add_smoothness_constraint",
     "ddsolve_add_antenna_constraint", "ddsolve_add_reference_antenna_constraint",
     "ddsolve_clear_constraints", "ddsolve_correct_and_subtract",
+    "ddsolve_check_wait_limit",
 )
 
 
@@ -118,6 +119,7 @@ def lib():
         L.ddsolve_set_tuning.argtypes = [vp, u32, u32]
         L.ddsolve_time_stream_kernel.argtypes = [vp, u32,
                                                  ctypes.POINTER(ctypes.c_float)]
+        L.ddsolve_check_wait_limit.argtypes = [vp, u32]
         L.ddsolve_last_launch_count.argtypes = [vp]
         L.ddsolve_last_launch_count.restype = u64
         _lib = L

@@ -489,6 +489,16 @@ DDSOLVE_API int ddsolve_perform_iteration_noalloc(
     const uint32_t* antenna1, const uint32_t* antenna2,
     const double* solutions, double* next_solutions, void* stream);
 
+/* Self-check of the failure detection of a solve (no reference counterpart):
+ * the pipelined path's CTAs wait for one another, every wait within a limit of
+ * 4 s, after which the solve ends with DDSOLVE_E_TIMEOUT. This call runs the
+ * context's solve on its uploaded data, from solutions of 1 + i, with a limit
+ * of wait_ms and a grid barrier that expects one arrival more than there are
+ * CTAs, so that its first wait runs out. Returns DDSOLVE_E_TIMEOUT when the
+ * solve has ended so, as it must; DDSOLVE_E_UNSUPPORTED where a solve has no
+ * such wait (other plans, device constraints). The context stays usable. */
+DDSOLVE_API int ddsolve_check_wait_limit(ddsolve_ctx* ctx, uint32_t wait_ms);
+
 /* Number of kernel launches issued by the last ddsolve_solve call (an
  * unconstrained solve on the pipelined path runs up to 64 iterations in one). */
 DDSOLVE_API uint64_t ddsolve_last_launch_count(const ddsolve_ctx* ctx);

@@ -62,3 +62,34 @@ def test_non_finite_blocks_of_every_interval(built, n_dir, n_st, n_intervals):
         np.testing.assert_allclose(got[-1, 1 + g], ref[-1, 1 + g], rtol=RTOL_SOLVE)
         ok = np.arange(n_st) != 1 + g
         assert H.max_rel_diff(got[:, ok], ref[:, ok]) < RTOL_SOLVE
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_dir,n_intervals,max_iterations", [(2, 1, 70), (2, 3, 5), (21, 1, 5)])
+def test_wait_limit_ends_the_solve(built, n_dir, n_intervals, max_iterations):
+    """A grid barrier that is never complete: the solve ends with an error
+    within the limit of its waits, the launches queued behind it do nothing,
+    and the next solve on the context is what it was before (the same bits:
+    every sum has a fixed order)."""
+    from dp3_b200 import ddsolve
+    n_cb = 2
+    obs = H.small_observation(n_stations=12, n_directions=n_dir, n_channels=4, n_cb=n_cb,
+                              n_times=2, seed=3, n_sources=2)
+    st = ddsolve.default_settings()
+    st.max_iterations, st.accuracy, st.detect_stalling = max_iterations, 1e-30, 0
+    ctx = ddsolve.Context(12, [1] * n_dir, n_intervals * n_cb, 2, 2)
+    ctx.set_settings(st)
+    if n_intervals > 1:
+        ctx.set_intervals([g * n_cb for g in range(n_intervals + 1)])
+    for cb in range(n_intervals * n_cb):
+        ctx.set_channel_block_regular(cb, 2, obs.cfg.n_baselines, obs.cfg.cb_channels[cb % n_cb],
+                                      obs.data[cb % n_cb], obs.model[cb % n_cb], obs.antenna1,
+                                      obs.antenna2)
+    solve = ctx.solve_batch if n_intervals > 1 else ctx.solve
+    before = np.ones((n_intervals * n_cb, 12, n_dir, 2), np.complex128)
+    solve(before)
+    assert ddsolve.lib().ddsolve_check_wait_limit(ctx._h, 20) == 5
+    after = np.ones_like(before)
+    solve(after)
+    ctx.close()
+    np.testing.assert_array_equal(after, before)
