@@ -61,6 +61,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
 constexpr uint32_t kMaxAntennas = 65535;
+constexpr size_t kB200BlockSmem = 227 * 1024;  // shared memory a block may ask for
 
 // ---------------------------------------------------------------------------
 // Device-side plan structures
@@ -4287,34 +4288,44 @@ struct PipeLayout {
   uint32_t stages;  // as many as fit, 0 when not even two do
   size_t stage_bytes;
 };
-PipeLayout MakePipeLayout(const ddsolve_ctx* ctx, uint32_t ng, uint32_t warps, uint32_t n_gbuf,
+
+// What the choice of the kernel and its layout depend on.
+struct PipeDims {
+  uint32_t n_ant, n_dir, n_corr, n_pol;
+  size_t max_smem;  // dynamic shared memory a block may ask for
+};
+PipeDims DimsOf(const ddsolve_ctx* ctx) {
+  return {ctx->n_ant, ctx->n_dir, ctx->n_corr, ctx->n_pol, ctx->max_smem};
+}
+
+PipeLayout MakePipeLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, uint32_t n_gbuf,
                           bool stage_q) {
   auto align = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
-  const size_t runs = warps * 32 / ng, n_dir = ctx->n_dir, n_corr = ctx->n_corr;
+  const size_t runs = warps * 32 / ng, n_dir = dims.n_dir, n_corr = dims.n_corr;
   const size_t table_f2 =
-      (size_t(ctx->n_ant) * PipeGainStride(ctx->n_dir, ctx->n_pol) + 1) & ~size_t(1);
+      (size_t(dims.n_ant) * PipeGainStride(dims.n_dir, dims.n_pol) + 1) & ~size_t(1);
   PipeLayout l{};
   size_t off = align(sizeof(PipeShared), 128);
   l.off_acc = uint32_t(off);
-  off += PipeAccFloats(ctx->n_ant, ctx->n_dir, ctx->n_pol) * 4;
+  off += PipeAccFloats(dims.n_ant, dims.n_dir, dims.n_pol) * 4;
   l.off_gtab = uint32_t(off);
   off += n_gbuf * table_f2 * 8;
   l.off_stg = uint32_t(off);
   const size_t staged = std::min<size_t>(n_dir, StageDirs(int(warps)) * ng);
-  off += staged * runs * (ctx->n_pol == 1 ? 1 : n_corr) * 8;
+  off += staged * runs * (dims.n_pol == 1 ? 1 : n_corr) * 8;
   l.off_q = uint32_t(off);
-  if (ctx->n_pol == 1)
+  if (dims.n_pol == 1)
     off += staged * runs * 4;
   else if (stage_q)
     off += staged * n_corr * runs * 4;
   l.off_meta = uint32_t(off = align(off, 16));
-  l.meta_words = MetaWords(uint32_t(runs), ctx->n_ant);
+  l.meta_words = MetaWords(uint32_t(runs), dims.n_ant);
   off += 2 * size_t(l.meta_words) * 4;
   off = align(off, 128);
-  if (off >= ctx->max_smem) return l;
+  if (off >= dims.max_smem) return l;
   l.off_stages = uint32_t(off);
   l.stage_bytes = runs * (1 + n_dir) * n_corr * 8;
-  const size_t fit = (ctx->max_smem - off) / l.stage_bytes;
+  const size_t fit = (dims.max_smem - off) / l.stage_bytes;
   l.stages = fit < 2 ? 0u : uint32_t(std::min<size_t>(fit, kPipeMaxStages));
   return l;
 }
@@ -4328,16 +4339,16 @@ PipeLayout MakePipeLayout(const ddsolve_ctx* ctx, uint32_t ng, uint32_t warps, u
 // 40 directions on 62 stations (twelve shuffles a row for five directions).
 // Fewer than three stages cost more than the shuffles of more lanes; from three
 // on the fewer lanes win (512 stations, 5 directions: 263 us against 320).
-const KernelEntry* FindPipeKernel(const ddsolve_ctx* ctx) {
+const KernelEntry* FindPipeKernel(const PipeDims& dims) {
   const KernelEntry* best = nullptr;
   uint32_t best_stages = 0;
   for (uint32_t ng = 1; ng <= 8 && best_stages < 3; ng *= 2) {
-    const uint32_t dpl = (ctx->n_dir + ng - 1) / ng;
+    const uint32_t dpl = (dims.n_dir + ng - 1) / ng;
     for (const KernelEntry& e : PipeKernels()) {
-      if (e.ncorr != int(ctx->n_corr) || e.npol != int(ctx->n_pol) || e.dmax != int(dpl) ||
+      if (e.ncorr != int(dims.n_corr) || e.npol != int(dims.n_pol) || e.dmax != int(dpl) ||
           e.ng != int(ng))
         continue;
-      const uint32_t stages = MakePipeLayout(ctx, ng, uint32_t(e.warps), 1, true).stages;
+      const uint32_t stages = MakePipeLayout(dims, ng, uint32_t(e.warps), 1, true).stages;
       if (stages <= best_stages) continue;
       best = &e;
       best_stages = stages;
@@ -4371,11 +4382,14 @@ int CheckDims(const ddsolve_dims* dims) {
 // runs, a multiple of 4; a short remainder tile would stream its rows at a
 // fraction of the bytes per pipeline stage). With eight lanes per run a
 // quarter warp reads four runs of two direction rows: their rows lie in
-// distinct shared-memory banks when the tile is 4 mod 8 runs wide.
-uint32_t LayoutTileRuns(const ddsolve_ctx* ctx, uint32_t R) {
-  const KernelEntry* e = FindPipeKernel(ctx);
+// distinct shared-memory banks when the tile is 4 mod 8 runs wide. Where no
+// pipelined kernel runs, tiles of at most kStreamTileRuns (the full-Jones
+// solve of 62 stations and 4 directions: 15.59 ms with 352, 15.54 with 224).
+constexpr uint32_t kStreamTileRuns = 224;
+uint32_t LayoutTileRuns(const PipeDims& dims, uint32_t R) {
+  const KernelEntry* e = FindPipeKernel(dims);
   const uint32_t ng = e ? uint32_t(e->ng) : 1u;
-  const uint32_t max_runs = uint32_t(e ? e->warps : kWarps) * 32 / ng;
+  const uint32_t max_runs = e ? uint32_t(e->warps) * 32 / ng : kStreamTileRuns;
   if (R == 0) return max_runs;
   const uint32_t n_tiles = (R + max_runs - 1) / max_runs;
   const uint32_t w = ((R + n_tiles - 1) / n_tiles + 3u) & ~3u;
@@ -4604,7 +4618,7 @@ int UploadAndPack(ddsolve_ctx* ctx, ChannelBlockStore& cb, const StageFn& stage,
   std::vector<PackSlab> ps(cb.slabs.size());
   for (size_t i = 0; i < cb.slabs.size(); ++i) {
     HostSlab& s = cb.slabs[i];
-    s.W = LayoutTileRuns(ctx, s.R);
+    s.W = LayoutTileRuns(DimsOf(ctx), s.R);
     ps[i] = PackSlab{s.elem_off, s.src_base, s.tstride, s.T, s.L, s.R, s.run_off, s.W};
   }
   char* st = ctx->staging.as<char>();
@@ -4967,9 +4981,9 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   // a pass.
   const uint32_t warps = uint32_t(ctx->pipe_entry->warps);
   uint32_t n_gbuf = ctx->tune_gbuf == 1 ? 1u : 2u;
-  PipeLayout lay = MakePipeLayout(ctx, ctx->pipe_ng, warps, n_gbuf, !use_powers);
+  PipeLayout lay = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, n_gbuf, !use_powers);
   if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 4u)) {
-    const PipeLayout one = MakePipeLayout(ctx, ctx->pipe_ng, warps, 1, !use_powers);
+    const PipeLayout one = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, 1, !use_powers);
     if (one.stages > lay.stages) {
       n_gbuf = 1;
       lay = one;
@@ -5201,7 +5215,7 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   ctx->pipe_ng = 1;
   if (allow_pipe && ctx->tune_ng == 0 && ctx->tune_pipe != 0 &&
       (ctx->n_corr == 2 || ctx->n_corr == 4) && !std::getenv("DDSOLVE_NO_PIPE")) {
-    const KernelEntry* pe = FindPipeKernel(ctx);
+    const KernelEntry* pe = FindPipeKernel(DimsOf(ctx));
     if (pe) {
       ctx->use_pipe = true;
       ctx->pipe_entry = pe;
@@ -5926,6 +5940,23 @@ void ddsolve_default_settings(ddsolve_settings* s) {
   s->detect_stalling = 1;
   s->step_diff_sigma = 0.1;
   s->phase_only = 0;
+}
+
+int ddsolve_describe_layout(const ddsolve_dims* dims, ddsolve_layout* layout) {
+  if (!layout) return DDSOLVE_E_INVALID;
+  const int dc = CheckDims(dims);
+  if (dc != DDSOLVE_OK) return dc;
+  const PipeDims d{dims->n_antennas, dims->n_directions, dims->n_correlations,
+                   dims->n_solution_polarizations, kB200BlockSmem};
+  *layout = {};
+  layout->tile_runs = LayoutTileRuns(d, 0);
+  if (const KernelEntry* e = FindPipeKernel(d)) {
+    layout->pipelined = 1;
+    layout->lanes_per_run = uint32_t(e->ng);
+    layout->directions_per_lane = uint32_t(e->dmax);
+    layout->stages = MakePipeLayout(d, uint32_t(e->ng), uint32_t(e->warps), 1, true).stages;
+  }
+  return DDSOLVE_OK;
 }
 
 int ddsolve_create(const ddsolve_dims* dims, int device, ddsolve_ctx** out) {
@@ -7202,7 +7233,7 @@ int ddsolve_autotune(ddsolve_ctx* ctx, uint32_t launches, ddsolve_tuning* chosen
   }
   // candidates: pipe_kernel plan variants, then stream_kernel lane groups
   std::vector<ddsolve_tuning> cands;
-  const bool pipe_ok = (ctx->n_corr == 2 || ctx->n_corr == 4) && FindPipeKernel(ctx);
+  const bool pipe_ok = (ctx->n_corr == 2 || ctx->n_corr == 4) && FindPipeKernel(DimsOf(ctx));
   if (pipe_ok)
     for (int32_t powers : {0, 1})
       for (uint32_t gbuf : {1u, 2u})

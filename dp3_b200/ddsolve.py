@@ -29,7 +29,7 @@ EXPORTED_SYMBOLS = (
     "ddsolve_set_interval_buffers", "ddsolve_add_smoothness_constraint",
     "ddsolve_add_antenna_constraint", "ddsolve_add_reference_antenna_constraint",
     "ddsolve_clear_constraints", "ddsolve_correct_and_subtract",
-    "ddsolve_check_wait_limit",
+    "ddsolve_check_wait_limit", "ddsolve_describe_layout",
 )
 
 
@@ -40,6 +40,14 @@ class Dims(ctypes.Structure):
                 ("n_correlations", ctypes.c_uint32),
                 ("n_solution_polarizations", ctypes.c_uint32),
                 ("n_solutions_per_direction", ctypes.POINTER(ctypes.c_uint32))]
+
+
+class Layout(ctypes.Structure):
+    _fields_ = [("pipelined", ctypes.c_int32),
+                ("tile_runs", ctypes.c_uint32),
+                ("lanes_per_run", ctypes.c_uint32),
+                ("directions_per_lane", ctypes.c_uint32),
+                ("stages", ctypes.c_uint32)]
 
 
 class Settings(ctypes.Structure):
@@ -120,10 +128,23 @@ def lib():
         L.ddsolve_time_stream_kernel.argtypes = [vp, u32,
                                                  ctypes.POINTER(ctypes.c_float)]
         L.ddsolve_check_wait_limit.argtypes = [vp, u32]
+        L.ddsolve_describe_layout.argtypes = [ctypes.POINTER(Dims), ctypes.POINTER(Layout)]
         L.ddsolve_last_launch_count.argtypes = [vp]
         L.ddsolve_last_launch_count.restype = u64
         _lib = L
     return _lib
+
+
+def describe_layout(n_antennas, n_directions, n_correlations, n_polarizations):
+    """The layout and kernel that these dimensions get (needs no GPU)."""
+    nspd = (ctypes.c_uint32 * n_directions)(*([1] * n_directions))
+    dims = Dims(n_antennas, n_directions, 1, n_correlations, n_polarizations,
+                ctypes.cast(nspd, ctypes.POINTER(ctypes.c_uint32)))
+    layout = Layout()
+    rc = lib().ddsolve_describe_layout(ctypes.byref(dims), ctypes.byref(layout))
+    if rc != DDSOLVE_OK:
+        raise RuntimeError(f"ddsolve_describe_layout: {ERRORS.get(rc, rc)}")
+    return layout
 
 
 def default_settings():

@@ -423,6 +423,18 @@ typedef struct {
 DDSOLVE_API int ddsolve_get_tuning(const ddsolve_ctx* ctx, ddsolve_tuning* tuning);
 DDSOLVE_API int ddsolve_set_plan_tuning(ddsolve_ctx* ctx, const ddsolve_tuning* tuning);
 
+/* The packed layout and the kernel that a context of these dimensions gets on
+ * a B200, before any data is uploaded; needs no GPU. */
+typedef struct {
+  int32_t pipelined;            /* 1: pipe_kernel, 0: the other streaming kernels */
+  uint32_t tile_runs;           /* baselines per tile of the layout, at most */
+  uint32_t lanes_per_run;       /* pipe_kernel: threads that share a baseline, */
+  uint32_t directions_per_lane; /* the directions of each, */
+  uint32_t stages;              /* and the depth of its bulk-copy ring */
+} ddsolve_layout;
+
+DDSOLVE_API int ddsolve_describe_layout(const ddsolve_dims* dims, ddsolve_layout* layout);
+
 /* Autotuner: on the uploaded data, times every applicable plan variant
  * (pipe_kernel with model powers on / off, one or two gain-table buffers,
  * all or three ring stages; stream_kernel with 1..32 lanes per run) over
