@@ -8,6 +8,8 @@
 Both are built with explicit nvcc / g++ command lines (no JIT cache), so the
 shared objects live next to the sources and travel with the repository tree.
 """
+import concurrent.futures
+import glob
 import os
 import subprocess
 import sys
@@ -20,6 +22,8 @@ INCLUDE = os.path.join(ROOT, "include")
 SOLVER_SO = os.path.join(HERE, "libddsolve_b200.so")
 SYNTH_SO = os.path.join(HERE, "libdp3b200_synth.so")
 WARM_SO = os.path.join(HERE, "libddwarm_b200.so")
+
+OBJ_DIR = os.path.join(HERE, "_build")  # the solver's object files
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -37,20 +41,34 @@ def _run(cmd):
     subprocess.check_call(cmd)
 
 
-def build_solver(force=False, verbose_ptxas=False):
-    srcs = [os.path.join(CSRC, "ddsolve.cu"),
-            os.path.join(INCLUDE, "ddsolve_b200.h")]
-    if not force and not _stale(SOLVER_SO, srcs):
-        return SOLVER_SO
-    # --split-compile=0: the device code of the many pipe_kernel variants is
-    # optimised on every core (16 minutes of compilation in under five on four)
-    cmd = [NVCC, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-shared",
-           "--split-compile=0",
+def solver_sources():
+    """Source files of the solver, each compiled to an object of its own:
+    ddsolve.cu and the variants of pipe_kernel."""
+    return sorted(glob.glob(os.path.join(CSRC, "pipe_*.cu"))) + [os.path.join(CSRC, "ddsolve.cu")]
+
+
+def solver_command(src, obj, verbose_ptxas=False):
+    cmd = [NVCC, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-c",
            "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
-           "-I", INCLUDE, "-o", SOLVER_SO, srcs[0], "-lcudart"]
+           "-I", INCLUDE, "-o", obj, src]
     if verbose_ptxas:
         cmd.insert(1, "-Xptxas=-v")
-    _run(cmd)
+    return cmd
+
+
+def build_solver(force=False, verbose_ptxas=False):
+    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + [
+        os.path.join(CSRC, "pipe_registry.h"), os.path.join(INCLUDE, "ddsolve_b200.h")]
+    srcs = solver_sources()
+    if not force and not _stale(SOLVER_SO, srcs + headers):
+        return SOLVER_SO
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    objs = [os.path.join(OBJ_DIR, os.path.basename(s) + ".o") for s in srcs]
+    todo = [solver_command(s, o, verbose_ptxas) for s, o in zip(srcs, objs)
+            if force or _stale(o, [s] + headers)]
+    with concurrent.futures.ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        list(pool.map(_run, todo))
+    _run([NVCC, *ARCH, "-shared", "-o", SOLVER_SO, *objs, "-lcudart"])
     return SOLVER_SO
 
 
