@@ -2035,6 +2035,7 @@ struct ddsolve_ctx {
   const void* pipe_fn = nullptr;
   size_t pipe_smem = 0;
   uint32_t pipe_stages = 0, acc_stride = 0, gain_stride = 0;
+  bool pipe_hold = false;  // PipeLayout::hold
   uint32_t pipe_ng = 1;  // lanes per run of the chosen pipe_kernel
   DevBuf d_cb_done /* new non-finite flags */, d_cb_flag, d_cb_avg, d_counters;
   DevBuf d_frags, d_cta_frag_off, d_tables, d_tab_cb, d_tab_sol, d_tab_off, d_tab_ent;
@@ -2246,8 +2247,8 @@ uint32_t PipeAccStride(uint32_t n_dir, uint32_t n_pol) {
   return s;
 }
 // Floats of an accumulator table and partial slot, whole 16-byte groups.
-size_t PipeAccFloats(uint32_t n_ant, uint32_t n_dir, uint32_t n_pol) {
-  return (size_t(n_ant) * PipeAccStride(n_dir, n_pol) + 3) & ~size_t(3);
+size_t PipeAccFloats(uint32_t n_ant, uint32_t acc_stride) {
+  return (size_t(n_ant) * acc_stride + 3) & ~size_t(3);
 }
 uint32_t PipeGainStride(uint32_t n_dir, uint32_t n_pol) {
   uint32_t s = n_dir * n_pol;
@@ -2263,8 +2264,9 @@ uint32_t PipeGainStride(uint32_t n_dir, uint32_t n_pol) {
 // summed in the row loop), two antenna buffers, the ring.
 struct PipeLayout {
   uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
-  uint32_t meta_words;
+  uint32_t meta_words, acc_stride;
   uint32_t stages;  // as many as fit, 0 when not even two do
+  bool hold;        // wide variant: sums staged in the ring stage of a tile's last row
   size_t stage_bytes;
 };
 
@@ -2278,33 +2280,47 @@ PipeDims DimsOf(const ddsolve_ctx* ctx) {
 }
 
 PipeLayout MakePipeLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, uint32_t n_gbuf,
-                          bool stage_q) {
+                          bool stage_q, bool hold = false) {
   auto align = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
   const size_t runs = warps * 32 / ng, n_dir = dims.n_dir, n_corr = dims.n_corr;
   const size_t table_f2 =
       (size_t(dims.n_ant) * PipeGainStride(dims.n_dir, dims.n_pol) + 1) & ~size_t(1);
   PipeLayout l{};
+  l.hold = hold;
+  // (where every byte counts, one polarization's rows at any even stride)
+  l.acc_stride = hold && dims.n_pol == 1 ? (dims.n_dir * 3 + 1) & ~1u
+                                         : PipeAccStride(dims.n_dir, dims.n_pol);
   size_t off = align(sizeof(PipeShared), 128);
   l.off_acc = uint32_t(off);
-  off += PipeAccFloats(dims.n_ant, dims.n_dir, dims.n_pol) * 4;
+  off += PipeAccFloats(dims.n_ant, l.acc_stride) * 4;
   l.off_gtab = uint32_t(off);
   off += n_gbuf * table_f2 * 8;
-  l.off_stg = uint32_t(off);
-  const size_t staged = std::min<size_t>(n_dir, StageDirs(int(warps)) * ng);
-  off += staged * runs * (dims.n_pol == 1 ? 1 : n_corr) * 8;
-  l.off_q = uint32_t(off);
-  if (dims.n_pol == 1)
-    off += staged * runs * 4;
-  else if (stage_q)
-    off += staged * n_corr * runs * 4;
+  if (!hold) {
+    const int dpl = int((n_dir + ng - 1) / ng);
+    const size_t staged =
+        std::min<size_t>(n_dir, StageDirs(int(warps), dpl, int(dims.n_pol), stage_q) * ng);
+    l.off_stg = uint32_t(off);
+    off += StagedBytes(uint32_t(staged), uint32_t(runs), dims.n_corr, dims.n_pol);
+    l.off_q = uint32_t(off);
+    if (dims.n_pol == 1)
+      off += staged * runs * 4;
+    else if (stage_q)
+      off += staged * n_corr * runs * 4;
+  }
   l.off_meta = uint32_t(off = align(off, 16));
   l.meta_words = MetaWords(uint32_t(runs), dims.n_ant);
   off += 2 * size_t(l.meta_words) * 4;
   off = align(off, 128);
-  if (off >= dims.max_smem) return l;
-  l.off_stages = uint32_t(off);
   l.stage_bytes = runs * (1 + n_dir) * n_corr * 8;
-  const size_t fit = (dims.max_smem - off) / l.stage_bytes;
+  const size_t fit = off < dims.max_smem ? (dims.max_smem - off) / l.stage_bytes : 0;
+  // A deeper ring rather than a staging area where that leaves fewer than
+  // three stages: 256 stations, 16 directions, two stages and an area 211 us a
+  // pass, three without 178; 80 stations, 40 directions 92 and 93.
+  if (fit < 3 && !hold && warps == kWideWarps) {
+    const PipeLayout h = MakePipeLayout(dims, ng, warps, n_gbuf, stage_q, true);
+    if (h.stages > (fit < 2 ? 0 : fit)) return h;
+  }
+  l.off_stages = uint32_t(off);
   l.stages = fit < 2 ? 0u : uint32_t(std::min<size_t>(fit, kPipeMaxStages));
   return l;
 }
@@ -2317,7 +2333,11 @@ PipeLayout MakePipeLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, uin
 // variant: eight lanes of 5 with kWarps measured 443 us a pass against 329 for
 // 40 directions on 62 stations (twelve shuffles a row for five directions).
 // Fewer than three stages cost more than the shuffles of more lanes; from three
-// on the fewer lanes win (512 stations, 5 directions: 263 us against 320).
+// on the fewer lanes win (512 stations, 5 directions: 263 us against 320). 13
+// to 20 directions take the wide variant, whose tiles have 56 runs, where the
+// 88-run tiles of kWarps leave two stages (140 stations, 20 directions: 198 ->
+// 173 us) or none (256 stations, 16 directions, otherwise on stream_kernel:
+// 338 -> 178 us; 512 stations, one polarization: 330 -> 202).
 const KernelEntry* FindPipeKernel(const PipeDims& dims) {
   const KernelEntry* best = nullptr;
   uint32_t best_stages = 0;
@@ -2328,7 +2348,7 @@ const KernelEntry* FindPipeKernel(const PipeDims& dims) {
           e.ng != int(ng))
         continue;
       const uint32_t stages = MakePipeLayout(dims, ng, uint32_t(e.warps), 1, true).stages;
-      if (stages <= best_stages) continue;
+      if (stages <= best_stages || best_stages >= 3) continue;
       best = &e;
       best_stages = stages;
     }
@@ -2852,10 +2872,19 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   }
   // Model powers are precomputed (one stage per tile and iteration) when the
   // tiles are deep enough in rows for that stage to cost less than the two
-  // multiply-adds per row, direction and correlation it replaces.
-  const bool use_powers =
+  // multiply-adds per row, direction and correlation it replaces. With up to
+  // kPipeDirs2 directions a lane and a ring of two stages, one of them held
+  // during a tile's reduction, it never does (280 stations, 16 directions, 16
+  // rows a tile: 257 us a pass with it, 246 without; 12 directions a lane: 89
+  // and 94).
+  bool use_powers =
       !std::getenv("DDSOLVE_NO_POWERS") && n_runs_all > 0 &&
       (ctx->tune_powers == 1 || (ctx->tune_powers < 0 && run_rows >= 16 * n_runs_all));
+  if (use_powers && ctx->tune_powers < 0 && ctx->dmax <= kPipeDirs2) {
+    const PipeLayout l = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng,
+                                        uint32_t(ctx->pipe_entry->warps), 1, false);
+    use_powers = !(l.hold && l.stages == 2);
+  }
   // ---- fragments: rows balanced over the CTAs ----
   // A row weighs its bytes; every fragment, whole tile or part of one, adds
   // its reduction: 2.3 us against 0.7 us for a 31 KB row (62 stations, 10
@@ -2963,7 +2992,7 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   PipeLayout lay = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, n_gbuf, !use_powers);
   if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 4u)) {
     const PipeLayout one = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, 1, !use_powers);
-    if (one.stages > lay.stages) {
+    if (one.stages > lay.stages || (one.stages == lay.stages && lay.hold && !one.hold)) {
       n_gbuf = 1;
       lay = one;
     }
@@ -2973,6 +3002,8 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   if (stages < 2)
     return ctx->Fail(DDSOLVE_E_UNSUPPORTED, "pipelined kernel does not fit in shared memory");
   ctx->n_gbuf = n_gbuf;
+  ctx->acc_stride = lay.acc_stride;
+  ctx->pipe_hold = lay.hold;
   ctx->off_acc = lay.off_acc;
   ctx->off_gtab = lay.off_gtab;
   ctx->off_stg = lay.off_stg;
@@ -3028,7 +3059,7 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
                                       ctx->stream));
   DDS_CHECK_CUDA(ctx, ctx->d_partials.Reserve(
                           std::max<size_t>(1, size_t(n_visits) *
-                                                  PipeAccFloats(n_ant, n_dir, ctx->n_pol)) *
+                                                  PipeAccFloats(n_ant, ctx->acc_stride)) *
                               4));
   // norm partials per CTA, or per chunk of several intervals
   {
@@ -3199,7 +3230,6 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
       ctx->use_pipe = true;
       ctx->pipe_entry = pe;
       ctx->pipe_ng = uint32_t(pe->ng);
-      ctx->acc_stride = PipeAccStride(ctx->n_dir, ctx->n_pol);
       ctx->gain_stride = PipeGainStride(ctx->n_dir, ctx->n_pol);
       ctx->dmax = uint32_t(pe->dmax);
       ctx->ng = 1;
@@ -3210,7 +3240,6 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   uint32_t runs_per_block = 0;
   if (ctx->use_pipe) {
     runs_per_block = uint32_t(ctx->pipe_entry->warps) * 32 / ctx->pipe_ng;
-    slot_floats = size_t(ctx->n_ant) * ctx->acc_stride;
   } else {
     // Kernel choice: ng lanes per run so that each lane handles at most the
     // preferred number of directions.
@@ -3484,7 +3513,7 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.acc_stride = ctx->acc_stride;
   p.gain_stride = ctx->gain_stride;
   p.stages = ctx->pipe_stages;
-  p.acc_floats = uint32_t(PipeAccFloats(ctx->n_ant, ctx->n_dir, ctx->n_pol));
+  p.acc_floats = uint32_t(PipeAccFloats(ctx->n_ant, ctx->acc_stride));
   p.metas = ctx->d_metas.as<uint32_t>();
   p.meta_words = ctx->meta_words;
   p.n_gbuf = ctx->n_gbuf;
@@ -3496,6 +3525,7 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.off_q = ctx->off_q;
   p.off_meta = ctx->off_meta;
   p.off_stages = ctx->off_stages;
+  p.hold = ctx->pipe_hold ? 1u : 0u;
   p.fin_lists = ctx->d_fin_lists.as<FinList>();
   p.fin_visits = ctx->d_fin_visits.as<uint32_t>();
   p.n_groups = ctx->n_groups;

@@ -27,11 +27,12 @@ void AddLanes(std::vector<KernelEntry>& k) {
   using D = std::make_integer_sequence<int, int(NC == 2 ? kPipeDirs2 : kPipeDirs4)>;
   (AddDirections<NC, NP, NG>(k, D{}), ...);
 }
-// Four lanes per run of more directions each, fewer warps.
+// Four lanes per run of 4 directions (13 in all) to 12 each, fewer warps.
+constexpr int kWideFrom = 4;
 template <int NP, int... DM>
 void AddWide(std::vector<KernelEntry>& k, std::integer_sequence<int, DM...>) {
-  (k.push_back(PipeEntry<2, NP, int(kPipeDirs2) + 1 + DM, 4, kWideWarps>()), ...);
+  (k.push_back(PipeEntry<2, NP, kWideFrom + DM, 4, kWideWarps>()), ...);
 }
-using WideDirections = std::make_integer_sequence<int, kPipeDirsWide - kPipeDirs2>;
+using WideDirections = std::make_integer_sequence<int, kPipeDirsWide - kWideFrom + 1>;
 
 }  // namespace

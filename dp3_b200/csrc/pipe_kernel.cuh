@@ -88,6 +88,7 @@ struct PipeParams {
   uint32_t power_floats;  // floats per tile in `powers`
   // shared-memory layout (byte offsets)
   uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
+  uint32_t hold;  // wide variant: no staging area (PipeLayout::hold)
   const FinList* fin_lists;    // [n_cb * n_sub]
   const uint32_t* fin_visits;
   uint32_t* cb_flag;     // channel block holds non-finite solutions
@@ -1196,9 +1197,21 @@ __device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, u
 // 43 -> 19 us.
 // SUMQ: the model powers are summed in the row loop (else precomputed).
 constexpr int kPairValues = 6;  // model values per lane up to which two rows fit its registers
-// Of a lane's directions, staged at a time: all, or three with more than
-// kPipeDirs2 * 4 directions (40 take 101 KB of accumulators and gains).
-__host__ __device__ constexpr int StageDirs(int warps) { return warps == kWideWarps ? 3 : 8; }
+// Of a lane's directions, staged at a time: all, or in the wide variant what
+// the ring stage of a tile's last row holds too, where the sums are staged when
+// a ring of three stages leaves no room for an area of their own
+// (PipeLayout::hold): all of up to five directions (P and Q of two
+// polarizations: half of them), three of more (40 directions take 101 KB of
+// accumulators and gains). 512 stations, 16 directions, one polarization, 8
+// rows a tile: 214 us a pass staged in two rounds, 202 in one.
+__host__ __device__ constexpr int StageDirs(int warps, int dpl, int npol, bool sumq) {
+  if (warps != kWideWarps) return 8;
+  return dpl > int(kPipeDirs2) ? 3 : npol == 1 || !sumq ? dpl : (dpl + 1) / 2;
+}
+__host__ __device__ constexpr uint32_t StagedBytes(uint32_t staged, uint32_t runs, uint32_t ncorr,
+                                                   uint32_t npol) {  // of P
+  return staged * runs * (npol == 1 ? 1u : ncorr) * 8u;
+}
 template <int NCORR, int NPOL, int DPL, int NG, bool SUMQ, int W>
 __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p) {
   static_assert(32 % NG == 0, "lanes per run must divide a warp");
@@ -1212,8 +1225,9 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
   uint64_t* mfree = sh.mfree;
   float* acc = reinterpret_cast<float*>(smem + p.off_acc);
   float2* gtab_buf = reinterpret_cast<float2*>(smem + p.off_gtab);
-  float4* stg = reinterpret_cast<float4*>(smem + p.off_stg);
-  float2* stg_q = reinterpret_cast<float2*>(smem + p.off_q);
+  constexpr int kStage = StageDirs(W, DPL, NPOL, SUMQ);
+  constexpr bool kMayHold = W == kWideWarps;
+  const bool hold = kMayHold && p.hold != 0;
   uint32_t* metas = reinterpret_cast<uint32_t*>(smem + p.off_meta);
   char* stages = reinterpret_cast<char*>(smem + p.off_stages);
   constexpr uint32_t E = NCORR * 8;  // bytes per visibility
@@ -1504,6 +1518,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
             G[k][c] = cmul_conj(ga[RowPol<NCORR, NPOL>(c)], gb[ColPol<NCORR, NPOL>(c)]);
         }
       }
+      uint32_t rr = 0;
       // NR rows at once: the dependent steps of one row (load, residual,
       // shuffles, sums) fill the latencies of the other's.
       auto rows = [&](auto nr) {
@@ -1617,12 +1632,12 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
             }
         }
         __syncwarp();
-        if (lane == 0) {
+        // (a held last row's stage is released after the reduction)
+        if (lane == 0 && !(hold && rr + NR == n_rows)) {
 #pragma unroll
           for (int i = 0; i < NR; ++i) MbarArrive(&empty[stage[i]]);
         }
       };
-      uint32_t rr = 0;
       if constexpr (DPL * NCORR <= kPairValues)
         if (S >= 4)  // (a shorter ring would run dry)
           for (; rr + 2 <= n_rows; rr += 2) rows(std::integral_constant<int, 2>{});
@@ -1635,6 +1650,17 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
       // barriers and no read-modify-write chains, whatever the runs' order.
       uint32_t q_src = 0;  // none, or at [dir][run][corr] (SUMQ: of the staged ones)
       uint32_t q_stage = 0;
+      const uint32_t held = st == 0 ? S - 1 : st - 1;  // the last row's stage
+      constexpr int kFewest = (DPL - 1) * NG + 1;  // directions of this variant
+      static_assert(!kMayHold || (kStage < DPL ? kStage * NG : kFewest) *
+                                         (NPOL == 1 ? 12 : SUMQ ? 12 * NCORR : 8 * NCORR) <=
+                                     (1 + kFewest) * int(E),
+                    "the staged sums must fit in a held stage");
+      const uint32_t stg_at =
+          hold ? SmemAddr(stages + held * stage_bytes) : SmemAddr(smem) + p.off_stg;
+      const uint32_t stg_q_at =
+          hold ? stg_at + StagedBytes(min(uint32_t(kStage * NG), n_dir), RUNS, NCORR, NPOL)
+               : SmemAddr(smem) + p.off_q;
       if (flags & kFragPower) {
         // the tile's precomputed model powers, in the stage after its rows
         q_stage = st;
@@ -1645,17 +1671,19 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
         }
         q_src = SmemAddr(stages + q_stage * stage_bytes);
       } else if (SUMQ) {
-        q_src = SmemAddr(stg_q);
+        q_src = stg_q_at;
       }
+      float4* const stg = SharedPtr<float4>(stg_at);
+      float2* const stg_q = SharedPtr<float2>(stg_q_at);
 #pragma unroll
-      for (int k0 = 0; k0 < DPL; k0 += StageDirs(W)) {
+      for (int k0 = 0; k0 < DPL; k0 += kStage) {
         ConsumerBarrier<W>();  // the previous reduction is complete everywhere
         if (active) {
 #pragma unroll
-          for (int k = k0; k < DPL && k < k0 + StageDirs(W); ++k) {
+          for (int k = k0; k < DPL && k < k0 + kStage; ++k) {
             const uint32_t j = g + (k - k0) * NG;  // staged direction k0 * NG + j
             if (k < DPL - 1 || last_mine) {
-if constexpr (NPOL == 1) {
+              if constexpr (NPOL == 1) {
                 float3 v = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < NCORR; ++c) {
@@ -1688,16 +1716,19 @@ if constexpr (NPOL == 1) {
         }
         ConsumerBarrier<W>();
         const uint32_t d0 = k0 * NG;
-        const uint32_t n_staged = min(uint32_t(StageDirs(W) * NG), n_dir - d0);
-        const uint32_t q_from = NPOL == 1          ? SmemAddr(stg_q)
+        const uint32_t n_staged = min(uint32_t(kStage * NG), n_dir - d0);
+        const uint32_t q_from = NPOL == 1          ? stg_q_at
                                 : q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4
                                                  : q_src;
-        GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), SmemAddr(stg), q_from,
+        GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), stg_at, q_from,
                                       SmemAddr(acc), ctid, n_dir, d0, n_staged, p.acc_stride,
                                       p.gain_stride);
       }
+      // (this thread's sums in the held stage, before a copy overwrites them)
+      if (hold) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
+        if (hold) MbarArrive(&empty[held]);
         if (flags & kFragPower) MbarArrive(&empty[q_stage]);
         MbarArrive(&mfree[nfrag & 1u]);
       }

@@ -18,7 +18,8 @@ struct KernelEntry {
   int warps = 0;                    // pipe_kernel: consumer warps
 };
 
-// Correlations and solution polarizations; Wide: with kWideWarps.
+// Correlations and solution polarizations; Wide: 13 directions and more, with
+// kWideWarps.
 void AddPipe22(std::vector<KernelEntry>& k);
 void AddPipe21(std::vector<KernelEntry>& k);
 void AddPipe42(std::vector<KernelEntry>& k);
