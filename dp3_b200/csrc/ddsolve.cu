@@ -2043,6 +2043,7 @@ struct ddsolve_ctx {
   uint32_t off_acc = 0, off_gtab = 0, off_stg = 0, off_q = 0, off_meta = 0, off_stages = 0;
   DevBuf d_metas;
   uint32_t n_ctas = 0, n_visits = 0, fin_blocks = 0;
+  double pass_bytes = 0.0;     // visibilities that a pass of pipe_kernel reads
   uint64_t wait_ns = kWaitNs;  // see PipeParams
   uint32_t arrive_extra = 0;
   // precomputed model powers (pipe_kernel), refreshed after every upload
@@ -2092,10 +2093,12 @@ struct ddsolve_ctx {
   // state, step magnitudes), copied before the call's single synchronization.
   struct HostStage {
     uint32_t counters[4];
+    volatile uint32_t stopped;  // written by the control step that ends a solve
     LoopState ls;
     double mags[1];  // [mags_cap]
   };
   HostStage* h_stage = nullptr;
+  cudaEvent_t launch_done[2] = {};  // the last two launches of a solve's passes
   size_t mags_cap = 0;
 
   int Fail(int code, const std::string& msg) {
@@ -2107,6 +2110,8 @@ struct ddsolve_ctx {
     if (graph) cudaGraphDestroy(graph);
     if (stream) cudaStreamDestroy(stream);
     if (h_stage) cudaFreeHost(h_stage);
+    for (cudaEvent_t ev : launch_done)
+      if (ev) cudaEventDestroy(ev);
     if (predict_copied) cudaEventDestroy(predict_copied);
     if (predict_host) cudaFreeHost(predict_host);
     if (small_host) cudaFreeHost(small_host);
@@ -2901,8 +2906,10 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   auto frag_cost = [&](const Tile&) { return reduce_bytes; };
   uint64_t total_rows = 0;
   double total_w = 0.0, max_one = 0.0;
+  ctx->pass_bytes = 0.0;
   for (const Tile& t : tiles) {
     total_rows += t.rows;
+    ctx->pass_bytes += double(t.rows) * t.n * (1 + n_dir) * ctx->elem_bytes;
     total_w += double(t.rows) * row_cost(t) + frag_cost(t);
     max_one = std::max(max_one, frag_cost(t) + row_cost(t));
   }
@@ -3549,6 +3556,7 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.counters = ctx->d_counters.as<uint32_t>();
   p.next_out = ctx->d_next.as<double2>();
   p.n_iters = 1;
+  p.host_stopped = nullptr;
   p.out_stride = 0;
   p.host_mode = host_mode ? 1 : 0;
   p.fin_mode = kFinFused;
@@ -3776,6 +3784,12 @@ int LaunchFullJones(ddsolve_ctx* ctx, bool host_mode, bool use_handle, bool with
   return DDSOLVE_OK;
 }
 
+// Passes of one launch of pipe_kernel (see kLaunchBytes).
+uint32_t PassesPerLaunch(const ddsolve_ctx* ctx) {
+  const double n = kLaunchBytes / std::max(ctx->pass_bytes, 1.0);
+  return n < 1.0 ? 1u : uint32_t(std::min<double>(n, kItersPerLaunch));
+}
+
 // `n_passes` (pipe_kernel, without constraints): passes of the one launch --
 // a solve's iterations until it stops, or in host mode a chain of
 // next-solutions passes into consecutive slots of `out_stride` values.
@@ -3790,6 +3804,8 @@ int LaunchIteration(ddsolve_ctx* ctx, bool host_mode, bool use_handle,
     if (constrained) pp.fin_mode = kFinStepOnly;
     pp.n_iters = constrained ? 1u : n_passes;
     pp.out_stride = out_stride;
+    // (a solve's own launches: a constrained solve's are kept in a graph)
+    if (!host_mode && !constrained) pp.host_stopped = &ctx->h_stage->stopped;
     void* args[] = {&pp};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctx->n_ctas);
@@ -4684,13 +4700,24 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
   DDS_CHECK_CUDA(ctx, ctx->ReserveStage(n_mags));
   bool staged = false;
   uint32_t solve_launches = 0;
-  if (in_kernel)
-    for (size_t left = n_mags; left > 0;) {
-      const uint32_t n = uint32_t(std::min<size_t>(left, kItersPerLaunch));
+  if (in_kernel) {
+    // Two launches are queued at a time: the GPU does not wait for the host,
+    // and when the solve stops early at most one launch finds nothing to do.
+    ctx->h_stage->stopped = 0u;
+    const uint32_t per_launch = PassesPerLaunch(ctx);
+    for (size_t left = n_mags; left > 0; ++solve_launches) {
+      cudaEvent_t& done = ctx->launch_done[solve_launches & 1u];
+      if (!done) DDS_CHECK_CUDA(ctx, cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+      if (solve_launches >= 2) {
+        DDS_CHECK_CUDA(ctx, cudaEventSynchronize(done));
+        if (ctx->h_stage->stopped) break;
+      }
+      const uint32_t n = uint32_t(std::min<size_t>(left, per_launch));
       if ((rc = LaunchIteration(ctx, false, false, false, n)) != DDSOLVE_OK) return rc;
       left -= n;
-      ++solve_launches;
+      if (left > 0) DDS_CHECK_CUDA(ctx, cudaEventRecord(done, ctx->stream));
     }
+  }
   if ((in_kernel || ctx->graph_ok) && n_groups == 1) {
     if (!in_kernel) DDS_CHECK_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
     DDS_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_stage->ls, ctx->d_state.ptr, sizeof(LoopState),
@@ -4740,7 +4767,7 @@ int SolveImpl(ddsolve_ctx* ctx, double* solutions, ddsolve_result* results,
     }
   }
   // pipe path: make_finite + build_tables (+ power_kernel) + the pipe_kernel
-  // launches (one per kItersPerLaunch iterations of the cap; with device
+  // launches (one per PassesPerLaunch iterations until it stops; with device
   // constraints one per iteration, and the constraints' kernels and the
   // assignment pass); else three kernels per iteration (full-Jones:
   // make_finite, the pass launches and the finalisation)
@@ -5032,16 +5059,17 @@ int ddsolve_perform_iterations(ddsolve_ctx* ctx, const double* start, uint32_t n
     DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
   }
   if (dev_in) ctx->d_sol.ptr = const_cast<double*>(start);
-  if (ctx->use_pipe) {  // the chain runs in the kernel, kItersPerLaunch passes per launch
+  if (ctx->use_pipe) {  // the chain runs in the kernel, several passes per launch
+    const uint32_t per_launch = PassesPerLaunch(ctx);
     if (ctx->use_powers && ctx->powers_dirty) ++launches;
     if ((rc = LaunchBuildTables(ctx)) != DDSOLVE_OK) return rc;
     if ((rc = LaunchPowers(ctx, false)) != DDSOLVE_OK) return rc;
     ++launches;
-    for (uint32_t k = 0; k < n_passes; k += kItersPerLaunch) {
+    for (uint32_t k = 0; k < n_passes; k += per_launch) {
       // later launches use the gain tables the one before left
       if (k > 0) ctx->d_sol.ptr = chain + bytes * (k - 1);
       ctx->d_next.ptr = chain + bytes * k;
-      if ((rc = LaunchIteration(ctx, true, false, false, std::min(n_passes - k, kItersPerLaunch),
+      if ((rc = LaunchIteration(ctx, true, false, false, std::min(n_passes - k, per_launch),
                                 n_sol)) != DDSOLVE_OK)
         return rc;
       ++launches;
@@ -5175,7 +5203,7 @@ int TimeIteration(ddsolve_ctx* ctx, uint32_t n, float* ms_out) {
   if ((rc = LaunchIteration(ctx, true, false, false)) != DDSOLVE_OK) return rc;  // warm-up
   DDS_CHECK_CUDA(ctx, cudaEventRecord(a, ctx->stream));
   // as a solve runs them: pipe_kernel's passes in one launch
-  const uint32_t per_launch = ctx->use_pipe ? std::min(n, kItersPerLaunch) : 1u;
+  const uint32_t per_launch = ctx->use_pipe ? std::min(n, PassesPerLaunch(ctx)) : 1u;
   for (uint32_t i = 0; i < n; i += per_launch)
     if ((rc = LaunchIteration(ctx, true, false, false, std::min(n - i, per_launch))) !=
         DDSOLVE_OK)

@@ -50,9 +50,14 @@ constexpr uint32_t kCounterWords = 128;
 constexpr size_t kCounterBytes = kCounterWords * 4;
 constexpr uint32_t kVerdictStop = 1u;  // the solve ends with this pass
 constexpr uint32_t kVerdictNear = 2u;  // it may end with the next one
-// Passes per launch at most: the launch ends within a bounded time, and other
-// contexts' kernels get the GPU.
+// Passes per launch at most, and the visibilities that its passes read (1.5 ms):
+// a launch holds every SM, and another context's kernels get the GPU between
+// two. 62 stations, 10 directions, 50 passes of 637 MB: a launch more adds 16 us
+// to a solve of 5.36 ms; with the next interval's upload and predict on a second
+// context an interval takes 8.7 to 9.5 ms with one launch a solve, 7.9 to 8.1
+// with 9 GB, 7.7 with 6 or 4 GB.
 constexpr uint32_t kItersPerLaunch = 64;
+constexpr double kLaunchBytes = 9e9;
 
 // The partial slots of one (channel block, sub-solution) in the finalisation:
 // a range of visits, or a list in fin_visits; its direction; and its gain-table
@@ -103,6 +108,7 @@ struct PipeParams {
   // output of pass k, which goes to next_out + k * out_stride.
   uint32_t n_iters;
   size_t out_stride;
+  volatile uint32_t* host_stopped;  // pinned host memory: set when a solve ends, or null
   int32_t host_mode;
   int32_t fin_mode;      // FinFused / FinStepOnly / FinAssignOnly
   const DevSettings* settings;
@@ -1021,6 +1027,7 @@ __device__ __forceinline__ bool EndPass(uint32_t smem_at, uint32_t it) {
         news == 2u ? kVerdictStop
                    : ControlPass<W, NPOL>(p, ctid, news != 0u, sh.sum, sh.cnt, sh.flag);
     if (ctid == 0) {
+      if ((v & kVerdictStop) && p.host_stopped) *p.host_stopped = 1u;
       p.counters[kCntVerdict] = v;
       StoreRelease(&p.counters[kCntEpoch], sh.epoch0 + it + 1);
     }
@@ -1257,7 +1264,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
     sh.stop = 0;
     sh.passes = 0;
     sh.params = p;
-    // A solve may be several launches (of kItersPerLaunch iterations, or the
+    // A solve may be several launches (of so many iterations, or the
     // unrolled body of a constrained solve's graph): a launch after the solve
     // has stopped, or after an error, does nothing. One thread looks: the
     // error may be flagged while it does, and the warps have to agree.

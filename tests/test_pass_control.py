@@ -93,3 +93,41 @@ def test_wait_limit_ends_the_solve(built, n_dir, n_intervals, max_iterations):
     solve(after)
     ctx.close()
     np.testing.assert_array_equal(after, before)
+
+
+@pytest.mark.gpu
+def test_launches_stop_with_the_solve(built):
+    """However many iterations are allowed, a solve that stops early has queued
+    at most one launch in vain (of 64 iterations each, for a small array)."""
+    obs = H.small_observation(n_stations=10, n_directions=2, n_channels=6, n_cb=2,
+                              n_times=2, seed=17)
+    prob = H.problem_from_observation(obs)
+    solver = H.make_solver(prob, max_iterations=6400, accuracy=1e-2, detect_stalling=False)
+    sol = H.unit_solutions(prob)
+    res = solver.Solve(H.solve_data_from_problem(prob), sol, 0.0)
+    assert res.iterations <= 64
+    assert solver._ctx.last_launch_count() <= 2 + 3, solver._ctx.last_launch_count()
+
+
+@pytest.mark.gpu
+def test_launches_are_bounded_in_time(built):
+    """Launches of many passes over a large interval would hold the GPU from
+    other contexts: 40 passes over 266 MB take two launches."""
+    from dp3_b200 import ddsolve
+    n_st, n_dir, n_cb, n_t, n_ch = 62, 10, 10, 10, 8
+    a1, a2 = (x.astype(np.uint32) for x in np.triu_indices(n_st, 1))
+    rng = np.random.default_rng(0)
+    model = rng.standard_normal((n_dir, n_t * len(a1) * n_ch, 2, 2), dtype=np.float32)
+    data = model.sum(0)
+    st = ddsolve.default_settings()
+    st.max_iterations, st.accuracy, st.detect_stalling = 40, 1e-30, 0
+    ctx = ddsolve.Context(n_st, [1] * n_dir, n_cb, 2, 2)
+    ctx.set_settings(st)
+    for cb in range(n_cb):
+        ctx.set_channel_block_regular(cb, n_t, len(a1), n_ch, data, model, a1, a2)
+    sol = np.full((n_cb, n_st, n_dir, 2), 1.1 + 0.1j)
+    assert ctx.solve(sol).iterations == 41  # the cap, not converged
+    assert 2 + 2 <= ctx.last_launch_count() <= 2 + 3
+    ctx.close()
+    # every block holds the same data (its rows split over other CTAs)
+    assert np.isfinite(sol).all() and H.max_rel_diff(sol[:1], sol[-1:]) < RTOL_SOLVE
