@@ -42,6 +42,10 @@ def built():
     return True
 
 
+ADAPTER_LIB = os.path.join(os.path.dirname(os.path.abspath(__file__)), "adapter", "_build",
+                           "libdp3_adapter_check.so")
+
+
 @pytest.hookimpl(wrapper=True)
 def pytest_runtest_call(item):
     """A test that compares with the reference's own solver is skipped where
@@ -53,6 +57,8 @@ def pytest_runtest_call(item):
     except ref_ffi.ReferenceMissing as e:
         pytest.skip(str(e))
     except OSError as e:
-        if ref_ffi.REFERENCE or "libdp3_adapter_check.so" not in str(e):
+        # (a library that is there and does not load fails)
+        if (ref_ffi.REFERENCE or os.path.basename(ADAPTER_LIB) not in str(e)
+                or os.path.exists(ADAPTER_LIB)):
             raise
         pytest.skip(str(e))
