@@ -2032,6 +2032,7 @@ struct ddsolve_ctx {
   // pipelined path (pipe_kernel): chosen when eligible
   bool use_pipe = false;
   const KernelEntry* pipe_entry = nullptr;
+  bool pass_loaded = false;  // its code is on the device
   const void* pipe_fn = nullptr;
   size_t pipe_smem = 0;
   uint32_t pipe_stages = 0, acc_stride = 0, gain_stride = 0;
@@ -2613,6 +2614,16 @@ int UploadAndPack(ddsolve_ctx* ctx, ChannelBlockStore& cb, const StageFn& stage,
                   bool models_in_place = false, int blk = -1) {
   const size_t E = ctx->elem_bytes;
   const size_t src_bytes = size_t(cb.n_vis) * E * (1 + ctx->n_dir);
+  // The kernel that will stream the block, loaded with the first upload rather
+  // than by the first solve (20 ms, once per process and group of variants).
+  if (!ctx->pass_loaded) {
+    if (const KernelEntry* e = FindPipeKernel(DimsOf(ctx))) {
+      cudaFuncAttributes attr;
+      DDS_CHECK_CUDA(ctx, cudaFuncGetAttributes(&attr, e->fn));
+      DDS_CHECK_CUDA(ctx, cudaFuncGetAttributes(&attr, e->fn_powers));
+    }
+    ctx->pass_loaded = true;
+  }
   if (blk < 0) DDS_CHECK_CUDA(ctx, ctx->staging.Reserve(src_bytes));  // else the block's own
   cb.vis.realloc_flag = cb.run_ant_dev.realloc_flag = false;
   DDS_CHECK_CUDA(ctx, cb.vis.Reserve(cb.n_elems * E * (1 + ctx->n_dir)));
