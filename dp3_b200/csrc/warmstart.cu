@@ -120,26 +120,14 @@ __host__ __device__ constexpr int ChunkGroups() {
   return R * (kKChunk / 8) / kGemmThreads;  // 16-byte groups per thread
 }
 
-// Row and 8-element K group of a thread's group g: along K for rows stored so
-// (16-byte loads), along the rows for transposed ones, whose 2-byte loads then
-// cover 32 neighbours. Either way 8 lanes store 128 contiguous bytes.
-template <int R>
-__device__ __forceinline__ void ChunkGroup(int g, int trans, int& r, int& kc) {
-  r = trans ? g % R : g >> 3;
-  kc = trans ? g / R : g & 7;
-}
-
-// Transposed operands of whole 8-row groups, 16-byte aligned: a thread reads 8
-// rows of n = 4 or 8 consecutive K at once (unit u: row group u % (R / 8), K
-// from n * (u / (R / 8)) on) and transposes them in registers. With 2-byte
-// loads a weight gradient of 1024 samples took 139 us; training on 6200 samples,
-// 3 epochs of 1024: 10.6 -> 6.2 ms.
+// Transposed operands (of whole 8-row groups, 16-byte aligned: Gemm): a thread
+// reads 8 rows of n = 4 or 8 consecutive K at once (unit u: row group
+// u % (R / 8), K from n * (u / (R / 8)) on) and transposes them in registers.
+// With 2-byte loads a weight gradient of 1024 samples took 139 us; training on
+// 6200 samples, 3 epochs of 1024: 10.6 -> 6.2 ms.
 template <int R>
 __host__ __device__ constexpr int TransUnitK() {
   return ChunkGroups<R>() < 8 ? ChunkGroups<R>() : 8;
-}
-__device__ __forceinline__ bool TransVector(int trans, int ld, int rows) {
-  return trans && (ld & 7) == 0 && (rows & 7) == 0;
 }
 
 // Global reads of a chunk (R rows x kKChunk of K) into registers, all of a
@@ -149,8 +137,7 @@ __device__ __forceinline__ void LoadChunkRegs(uint4 (&q)[ChunkGroups<R>()], cons
                                               int ld, int trans, int rows, int K, int row0,
                                               int k0) {
   static_assert((R * (kKChunk / 8)) % kGemmThreads == 0, "chunk groups must split evenly");
-  const bool fast = !trans && (ld & 7) == 0;
-  if (TransVector(trans, ld, rows)) {
+  if (trans) {
     constexpr int N = TransUnitK<R>();
 #pragma unroll
     for (int i = 0; i < ChunkGroups<R>(); ++i) {
@@ -162,10 +149,11 @@ __device__ __forceinline__ void LoadChunkRegs(uint4 (&q)[ChunkGroups<R>()], cons
     }
     return;
   }
+  const bool fast = (ld & 7) == 0;
 #pragma unroll
   for (int i = 0; i < ChunkGroups<R>(); ++i) {
-    int r, kc;
-    ChunkGroup<R>(threadIdx.x + i * kGemmThreads, trans, r, kc);
+    const int g = threadIdx.x + i * kGemmThreads;
+    const int r = g >> 3, kc = g & 7;
     const int row = row0 + r, k = k0 + kc * 8;
     if (fast && row < rows && k + 8 <= K) {
       q[i] = __ldg(reinterpret_cast<const uint4*>(src + size_t(row) * ld + k));
@@ -173,8 +161,7 @@ __device__ __forceinline__ void LoadChunkRegs(uint4 (&q)[ChunkGroups<R>()], cons
       uint16_t v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const bool in = row < rows && k + j < K;
-        v[j] = in ? (trans ? src[size_t(k + j) * ld + row] : src[size_t(row) * ld + k + j]) : 0;
+        v[j] = row < rows && k + j < K ? src[size_t(row) * ld + k + j] : 0;
       }
       memcpy(&q[i], v, 16);
     }
@@ -185,9 +172,9 @@ __device__ __forceinline__ void LoadChunkRegs(uint4 (&q)[ChunkGroups<R>()], cons
 // 8x8 core matrices of 128 contiguous bytes, K-adjacent cores 128 B apart,
 // 8-row groups 1024 B apart.
 template <int R>
-__device__ __forceinline__ void StoreChunkRegs(unsigned char* dst, int trans, int ld, int rows,
+__device__ __forceinline__ void StoreChunkRegs(unsigned char* dst, int trans,
                                                const uint4 (&q)[ChunkGroups<R>()]) {
-  if (TransVector(trans, ld, rows)) {
+  if (trans) {
     constexpr int N = TransUnitK<R>();
 #pragma unroll
     for (int i = 0; i < ChunkGroups<R>(); i += N) {
@@ -214,8 +201,8 @@ __device__ __forceinline__ void StoreChunkRegs(unsigned char* dst, int trans, in
   }
 #pragma unroll
   for (int i = 0; i < ChunkGroups<R>(); ++i) {
-    int r, kc;
-    ChunkGroup<R>(threadIdx.x + i * kGemmThreads, trans, r, kc);
+    const int g = threadIdx.x + i * kGemmThreads;
+    const int r = g >> 3, kc = g & 7;
     *reinterpret_cast<uint4*>(dst + ((r >> 3) * 8 + kc) * 128 + (r & 7) * 16) = q[i];
   }
 }
@@ -278,8 +265,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const GemmParams p) 
   for (int c = 0; c < n_chunks; ++c) {
     const int b = c & 1;
     if (c >= 2) MbarWait(&mbar[b], uint32_t((c - 2) >> 1) & 1u, p.error);  // chunk c - 2
-    StoreChunkRegs<kMTile>(a_buf + b * kABytes, p.a_trans, p.lda, p.M, qa);
-    StoreChunkRegs<NT>(b_buf + b * kBBytes, p.b_trans, p.ldb, p.N, qb);
+    StoreChunkRegs<kMTile>(a_buf + b * kABytes, p.a_trans, qa);
+    StoreChunkRegs<NT>(b_buf + b * kBBytes, p.b_trans, qb);
     if (c + 1 < n_chunks) {
       LoadChunkRegs<kMTile>(qa, p.a, p.lda, p.a_trans, p.M, p.K, m0, (c + 1) * kKChunk);
       LoadChunkRegs<NT>(qb, p.b, p.ldb, p.b_trans, p.N, p.K, n0, (c + 1) * kKChunk);
@@ -945,6 +932,9 @@ int Reserve(ddwarm_ctx* ctx, uint32_t rows) {
 int Gemm(ddwarm_ctx* ctx, const uint16_t* a, int lda, int a_trans, const uint16_t* b, int ldb,
          int b_trans, int M, int N, int K, void* c, int ldc, const float* bias,
          const uint16_t* mask, int epilogue) {
+  // what LoadChunkRegs takes for granted: every layer's sizes are multiples of 64
+  if ((a_trans && ((lda | M) & 7)) || (b_trans && ((ldb | N) & 7)))
+    return ctx->Fail(4, "a transposed operand is not made of whole 8-row groups");
   GemmParams p;
   p.a = a;
   p.b = b;
