@@ -25,8 +25,12 @@
 // visibilities: each model element is read from HBM exactly once per
 // iteration with full coalescing.
 //
-// Kernels per iteration (all on one stream, captured in one CUDA graph whose
-// while-node runs the whole iterate-until-converged loop):
+// A solve without device constraints runs on pipe_kernel (pipe_kernel.cuh)
+// where a variant fits: its passes, their finalisation and the stopping rule in
+// one launch, or a few. With device constraints each iteration is a pass of
+// pipe_kernel up to SolverBase::Step, the constraints' kernels and
+// assign_kernel, in a CUDA graph whose while-node runs the whole
+// iterate-until-converged loop. Elsewhere the graph's iteration is
 //   make_finite_kernel  SolverBase::MakeSolutionsFinite{1,2}Pol (only acts on
 //                       channel blocks flagged non-finite)
 //   stream_kernel       persistent: residual, per-direction P/Q sums, per-CTA
@@ -36,7 +40,8 @@
 //                       FP64 num/den + add-back, SolverBase::Step,
 //                       AssignSolutions norm, DetectStall and the stopping
 //                       rule (last block), which sets the graph's loop
-//                       condition.
+//                       condition;
+// full-Jones solutions have kernels of their own (fj_*).
 #include "ddsolve_b200.h"
 #include "pipe_kernel.cuh"
 #include "pipe_registry.h"
@@ -2761,8 +2766,6 @@ StageFn StagePredict(ddsolve_ctx* ctx, const ChannelBlockStore& cb, const float*
   };
 }
 
-constexpr int kPlanNoPipe = -1;  // BuildPipePlan: use the stream_kernel path
-
 // Appends the antenna block of a tile of n runs (antenna1 | antenna2 << 16
 // each; layout at kMetaRuns) to `metas`; first = its first word / 4. `at` is
 // scratch per antenna, zero between calls: an antenna's runs in the tile, then
@@ -2859,7 +2862,8 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
     // The tiles of the packed layout (LayoutTileRuns): a row of a tile is
     // one bulk copy.
     const uint32_t tile_runs = sd.W;
-    if (tile_runs == 0 || tile_runs > tile_max || (tile_runs & 3u)) return kPlanNoPipe;
+    if (tile_runs == 0 || tile_runs > tile_max || (tile_runs & 3u))
+      return ctx->Fail(DDSOLVE_E_STATE, "the packed tiles are not those of the pass");
     // A slab whose runs are those of an earlier one (the channel blocks and
     // time steps of a regular interval) shares its antenna blocks.
     constexpr size_t kNone = ~size_t(0);
@@ -2908,10 +2912,16 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   }
   // ---- fragments: rows balanced over the CTAs ----
   // A row weighs its bytes; every fragment, whole tile or part of one, adds
-  // its reduction: 2.3 us against 0.7 us for a 31 KB row (62 stations, 10
-  // directions), 4.5 us against 0.6 us for a 37 KB row in the wide variant. The
-  // least bound under which filling the CTAs in order covers all rows is
-  // found by bisection.
+  // its reduction: 2.7 us against 0.66 us for a 30 KB row (62 stations, 10
+  // directions), 5.4 us against 0.81 us for a 36 KB row of the wide variant (40
+  // directions), 120 and 245 KB. The weights are those of the shortest solves
+  // there (50 passes: 5.38, 5.36, 5.47 ms with 50, 100, 340 KB; 10 of the
+  // 40-direction interval: 3.86, 3.48, 3.53 ms with 170, 340, 450). Other shapes
+  // hardly depend on them: 512 stations and the wide variant's 13 to 20
+  // directions within 1 % from 50 to 340 KB, 24 and 30 directions within 3 % from
+  // 100 on; 48 directions would take 53 us with 50 KB instead of 56. The least
+  // bound under which filling the CTAs in order covers all rows is found by
+  // bisection.
   const double reduce_bytes = ctx->pipe_entry->warps == kWideWarps ? 340e3 : 100e3;
   auto row_cost = [&](const Tile& t) { return double(t.n) * (1 + n_dir) * ctx->elem_bytes + 1e3; };
   auto frag_cost = [&](const Tile&) { return reduce_bytes; };
@@ -3059,7 +3069,6 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   if ((rc = upload(ctx->d_frags, frags.data(), frags.size() * sizeof(Frag)))) return rc;
   if ((rc = upload(ctx->d_metas, metas.data(), metas.size() * 4))) return rc;
   if ((rc = upload(ctx->d_cta_frag_off, cta_off.data(), cta_off.size() * 4))) return rc;
-  if ((rc = upload(ctx->d_slab_sol, slab_sol.data(), slab_sol.size() * 4))) return rc;
   if ((rc = upload(ctx->d_fin_lists, fin_lists.data(), fin_lists.size() * sizeof(FinList))))
     return rc;
   if ((rc = upload(ctx->d_fin_visits, fin_visits.data(), fin_visits.size() * 4))) return rc;
@@ -3232,7 +3241,8 @@ int BuildFullJonesPlan(ddsolve_ctx* ctx) {
   return DDSOLVE_OK;
 }
 
-int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
+// The pipelined plan when it applies, else the stream_kernel plan.
+int BuildPlan(ddsolve_ctx* ctx) {
   for (uint32_t c = 0; c < ctx->n_cb; ++c)
     if (!ctx->cbs[c].set)
       return ctx->Fail(DDSOLVE_E_STATE,
@@ -3246,7 +3256,7 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   // shared memory allow it (and no lane groups were requested).
   ctx->use_pipe = false;
   ctx->pipe_ng = 1;
-  if (allow_pipe && ctx->tune_ng == 0 && ctx->tune_pipe != 0 &&
+  if (ctx->tune_ng == 0 && ctx->tune_pipe != 0 &&
       (ctx->n_corr == 2 || ctx->n_corr == 4) && !std::getenv("DDSOLVE_NO_PIPE")) {
     const KernelEntry* pe = FindPipeKernel(DimsOf(ctx));
     if (pe) {
@@ -3462,15 +3472,6 @@ int BuildPlanImpl(ddsolve_ctx* ctx, bool allow_pipe) {
   return DDSOLVE_OK;
 }
 
-// The pipelined plan when it applies (a lane-group pipe_kernel needs every
-// tile to take the direct reduction), else the stream_kernel plan.
-int BuildPlan(ddsolve_ctx* ctx) {
-  const int rc = BuildPlanImpl(ctx, true);
-  if (rc != kPlanNoPipe) return rc;
-  ctx->use_pipe = false;
-  return BuildPlanImpl(ctx, false);
-}
-
 StreamParams MakeStreamParams(ddsolve_ctx* ctx) {
   StreamParams p;
   p.slabs = ctx->d_slabs.as<SlabDesc>();
@@ -3522,7 +3523,6 @@ PipeParams MakePipeParams(ddsolve_ctx* ctx, bool host_mode, bool use_handle) {
   p.slabs = ctx->d_slabs.as<SlabDesc>();
   p.frags = ctx->d_frags.as<Frag>();
   p.cta_frag_off = ctx->d_cta_frag_off.as<uint32_t>();
-  p.slab_sol = ctx->d_slab_sol.as<uint32_t>();
   p.solutions = ctx->d_sol.as<double2>();
   p.partials = ctx->d_partials.as<float>();
   p.tables = ctx->d_tables.as<float2>();
@@ -5065,8 +5065,8 @@ int ddsolve_perform_iterations(ddsolve_ctx* ctx, const double* start, uint32_t n
     }
   } restore{ctx, ctx->d_sol.ptr, ctx->d_next.ptr};
   if (ctx->use_pipe) {
-    // Once per call (every pipe_kernel launch leaves its counters at zero;
-    // next-solutions passes use none of the solve's non-finite flags).
+    // Once per call (the counters go on from one pipe_kernel launch to the
+    // next; next-solutions passes use none of the solve's non-finite flags).
     DDS_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_counters.ptr, 0, kCounterBytes, ctx->stream));
   }
   if (dev_in) ctx->d_sol.ptr = const_cast<double*>(start);

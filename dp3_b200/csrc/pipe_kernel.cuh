@@ -11,25 +11,26 @@ namespace {
 // moves the (time, channel) rows of each tile from HBM into a ring of
 // shared-memory stages, one 1-D bulk copy per row (cp.async.bulk, completion
 // on an mbarrier, no multicast; the tile-packed slab layout makes a row of a
-// tile, data and every direction, contiguous). Seven consumer warps compute
-// the residual and the per-direction P/Q sums from shared memory, one lane per
-// run (or four lanes per run for 13-48 directions), and reduce each tile into
-// the CTA's shared-memory antenna accumulators in barrier-separated phases
-// over groups of runs with distinct antennas (runs are stored in
-// cyclic-diagonal order), or by a counting sort where a tile has no such
-// grouping. No shared-memory float atomics.
+// tile, data and every direction, contiguous). The consumer warps compute the
+// residual and the per-direction P/Q sums from shared memory, 1, 2, 4 or 8
+// lanes per run, and stage a tile's sums in shared memory; then a thread per
+// (antenna of the tile, group of directions) gathers that antenna's runs, in
+// the order of the tile's entry list, and updates the CTA's accumulators. Two
+// barriers per staging round, no shared-memory float atomics.
 //
-// The finalisation is fused: after a grid-wide arrival count, every CTA
-// finalises a slice of the (channel block, antenna, sub-solution) items (merge
-// of the partial slots, FP64 update, step, norm, non-finite detection for the
-// lazy MakeSolutionsFinite), interval by interval, and the last CTA to finish
-// runs the iteration control of every interval still going. One launch per
-// iteration. Every wait is bounded by a 4 s device timer; a timeout sets an
-// error flag that the host reports as DDSOLVE_E_TIMEOUT, and all later waits
-// of that CTA return at once so that the kernel still ends.
+// One launch runs several passes, up to a solve's stop. The finalisation is
+// part of it: after a grid-wide arrival count, every CTA finalises a share of
+// the (channel block, antenna, sub-solution) items (merge of the partial slots,
+// FP64 update, step, norm, gain tables, non-finite detection for the lazy
+// MakeSolutionsFinite); after a second one, the last CTA of the grid runs the
+// iteration control of every interval still going. Meanwhile the ring fills
+// with the next pass's rows, and the pass itself begins where its start cannot
+// depend on the verdict; it is given up before its finalisation when the solve
+// has stopped. Every wait is bounded by a device timer (4 s); when one runs out,
+// an error flag that the host reports as DDSOLVE_E_TIMEOUT ends the launch.
 // ---------------------------------------------------------------------------
 // Consumer warps of a CTA, beside one producer warp: kWarps (168 registers a
-// thread), or kWideWarps (255) for more than kPipeDirs2 * 4 directions.
+// thread), or kWideWarps (255) for 13 directions and more (FindPipeKernel).
 constexpr int kWarps = 11, kWideWarps = 7;
 // Directions per lane at most (2 and 4 correlations): gains, sums and the
 // model row of that many fit a thread's 168 registers; with kWideWarps, gains
@@ -73,7 +74,6 @@ struct PipeParams {
   const SlabDesc* slabs;
   const Frag* frags;
   const uint32_t* cta_frag_off;
-  const uint32_t* slab_sol;
   double2* solutions;
   float* partials;
   float2* tables;         // gain tables [n_tables][table_f2]
@@ -470,8 +470,8 @@ __device__ __forceinline__ void BlockNorm(int ctid, double& sum, uint32_t& cnt, 
     }
 }
 
-// An interval's loop state, read and written past L1: within one launch the
-// CTA that finishes a pass changes from pass to pass.
+// An interval's loop state, read and written past L1: within one launch one
+// CTA changes it, pass by pass, and every CTA reads it.
 __device__ __forceinline__ LoopState LoadState(const LoopState* s) {
   static_assert(sizeof(LoopState) % 8 == 0, "copied in 8-byte words");
   LoopState r;
@@ -638,8 +638,8 @@ __device__ __forceinline__ uint32_t ControlPass(const PipeParams& p, int ctid, b
 
 // Grid-wide finalisation of a pass of pipe_kernel, after the grid barrier:
 // the consumer threads of all CTAs take (channel block, antenna,
-// sub-solution) items, warp by warp over the CTAs, one round per independent
-// interval (one round for a single interval): fixed-order compensated merge
+// sub-solution) items, warp by warp over the CTAs (with several intervals, at
+// most 32 items of one interval a warp): fixed-order compensated merge
 // of the item's partial slots, FP64 add-back and division
 // (IterativeDiagonalSolver.cc:206-221, IterativeScalarSolver.cc:184-194),
 // SolverBase::Step (SolverBase.cc:88-158), the AssignSolutions norm
@@ -906,7 +906,6 @@ __global__ void build_tables_kernel(const double2* __restrict__ solutions,
   for (int q = 0; q < NPOL; ++q) dst[q] = make_float2(float(src[q].x), float(src[q].y));
 }
 
-// Launched cooperatively (all CTAs co-resident), one CTA per SM.
 // Model powers of the pipelined path: for every tile of runs, direction and
 // correlation, sum over the tile's (time, channel) rows of |M|^2. They depend
 // on the model alone, so they are computed once per upload instead of in
@@ -1193,15 +1192,14 @@ __device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, u
 // lane g of a run owns directions g, g + NG, ... (DPL of them); the residual
 // is the sum over the run's lanes (warp shuffles). NG = 1: one run per lane,
 // exactly DPL directions.
-// Bound: HBM (6.2 of 6.5 TB/s measured for a copy) while rows stream, and
-// latency in the end of a pass. 11 consumer warps of at most DPL = 5
-// directions a lane, in 168 registers without spills, cover each other's
-// latencies: a 31 KB row (62 stations, 10 directions) takes 0.6 us, the time
-// of its copy, a tile's reduction 2.0 us; 7 warps of up to 10 directions a lane
-// took 6.8 us for the reduction. One launch runs many passes, and the ring
-// fills with the next pass's rows while the grid finalises: 24 channel blocks
-// of 80 rows (240 channels, 8 times) 125 -> 103 us a pass, 12 blocks of 20 rows
-// 43 -> 19 us.
+// Launched cooperatively (all CTAs co-resident), one CTA per SM.
+// Bound: HBM while rows stream, and latency in the end of a pass. 11 consumer
+// warps of at most DPL = 5 directions a lane, in 168 registers, cover each
+// other's latencies: a 30 KB row (62 stations, 10 directions) takes 0.66 us, the
+// time of its copy, a tile's reduction 2.7 us; 7 warps of up to 10 directions a
+// lane took 6.8 us for the reduction. Several passes in one launch, the ring
+// filling while the grid finalises: 50 passes over 24 channel blocks of 80 rows
+// (240 channels, 8 times) 6.27 -> 5.41 ms, over 12 blocks of 20 rows 2.13 -> 1.05.
 // SUMQ: the model powers are summed in the row loop (else precomputed).
 constexpr int kPairValues = 6;  // model values per lane up to which two rows fit its registers
 // Of a lane's directions, staged at a time: all, or in the wide variant what
@@ -1402,7 +1400,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
           }
         }
         if (ok && (f.flags & kFragPower)) {
-          // one more stage: the tile's model powers [dir][corr][run]
+          // one more stage: the tile's model powers [dir][run][corr]
           if (!take_stage()) {
             ok = false;
             break;
