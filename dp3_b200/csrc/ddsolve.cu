@@ -714,9 +714,11 @@ __global__ void __launch_bounds__(kThreads)
 //   antenna 1: num += g_a2 P,        den += |g_a2|^2 Q  (segmented warp sum)
 //   antenna 2: num += g_a1 conj(P),  den += |g_a1|^2 Q  (shared atomics)
 // Accumulators: shared float [n_ant][n_dir][NPOL][3]; flushed per visit.
+// BLOCKS 1: compiled for one block per SM (registers instead of spills), for
+// passes with no more steps than SMs; 0: the compiler's choice.
 // ---------------------------------------------------------------------------
-template <int NCORR, int NPOL, int DMAX>
-__global__ void __launch_bounds__(kThreads)
+template <int NCORR, int NPOL, int DMAX, int BLOCKS = 0>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
     stream_kernel(const StreamParams p) {
   extern __shared__ float4 smem4[];
   float* acc = reinterpret_cast<float*>(smem4);
@@ -2205,13 +2207,20 @@ constexpr KernelEntry Entry() {
   return KernelEntry{NC, NP, DM,
                      reinterpret_cast<const void*>(&stream_kernel<NC, NP, DM>)};
 }
+// With the variant for one block per SM.
+template <int NC, int NP, int DM>
+KernelEntry EntryAlone() {
+  KernelEntry e = Entry<NC, NP, DM>();
+  e.fn_alone = reinterpret_cast<const void*>(&stream_kernel<NC, NP, DM, 1>);
+  return e;
+}
 
 const std::vector<KernelEntry>& Kernels() {
   static const std::vector<KernelEntry> k = {
       Entry<2, 2, 1>(), Entry<2, 2, 2>(), Entry<2, 2, 3>(), Entry<2, 2, 4>(),
       Entry<2, 2, 5>(), Entry<2, 2, 6>(), Entry<2, 2, 8>(),
       Entry<4, 2, 1>(), Entry<4, 2, 2>(), Entry<4, 2, 4>(),
-      Entry<1, 1, 1>(), Entry<1, 1, 2>(), Entry<1, 1, 4>(), Entry<1, 1, 8>(),
+      Entry<1, 1, 1>(), Entry<1, 1, 2>(), EntryAlone<1, 1, 4>(), EntryAlone<1, 1, 8>(),
       Entry<2, 1, 1>(), Entry<2, 1, 2>(), Entry<2, 1, 4>(), Entry<2, 1, 8>(),
       Entry<4, 1, 1>(), Entry<4, 1, 2>(), Entry<4, 1, 4>(),
   };
@@ -3296,18 +3305,23 @@ int BuildPlan(ddsolve_ctx* ctx) {
       return ctx->Fail(DDSOLVE_E_UNSUPPORTED, "too many directions for the kernel set");
     ctx->ng = ng;
     ctx->dmax = uint32_t(ke->dmax);
-    ctx->stream_fn = reinterpret_cast<StreamFn>(const_cast<void*>(ke->fn));
+    // One correlation: no more steps than SMs, so one block on each, without
+    // spills (62 stations, 12 blocks, 6 directions: 150 -> 137 us a pass); with
+    // more steps two blocks per SM take them sooner (10 directions: 70 -> 55 us).
+    size_t n_steps = 0;
+    for (const ChannelBlockStore& cb : ctx->cbs)
+      for (const HostSlab& s : cb.slabs) n_steps += (s.R + kThreads / ng - 1) / (kThreads / ng);
+    const void* fn = ke->fn_alone && n_steps <= size_t(ctx->n_sm) ? ke->fn_alone : ke->fn;
+    ctx->stream_fn = reinterpret_cast<StreamFn>(const_cast<void*>(fn));
     const size_t acc_n = size_t(ctx->n_ant) * ctx->n_dir * ctx->n_pol * 3;
     const size_t smem = ((acc_n + 3) & ~size_t(3)) * 4 +
                         size_t(ctx->n_ant) * ctx->n_dir * ctx->n_pol * 8;
     if (smem > size_t(max_optin))
       return ctx->Fail(DDSOLVE_E_UNSUPPORTED,
                        "antenna x direction accumulators exceed shared memory");
-    DDS_CHECK_CUDA(ctx, cudaFuncSetAttribute(ke->fn,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+    DDS_CHECK_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(smem)));
-    DDS_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                            &occ, ke->fn, kThreads, smem));
+    DDS_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kThreads, smem));
     if (occ < 1) return ctx->Fail(DDSOLVE_E_UNSUPPORTED, "stream kernel cannot launch");
     ctx->stream_smem = smem;
     runs_per_block = kThreads / ng;

@@ -16,6 +16,7 @@ struct KernelEntry {
   int ng = 1;  // pipe_kernel: lanes per run
   const void* fn_powers = nullptr;  // pipe_kernel: with precomputed model powers
   int warps = 0;                    // pipe_kernel: consumer warps
+  const void* fn_alone = nullptr;   // stream_kernel: for one block per SM
 };
 
 // Correlations and solution polarizations; Wide: 13 directions and more, with
