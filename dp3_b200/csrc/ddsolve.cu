@@ -2286,7 +2286,7 @@ struct PipeLayout {
   uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
   uint32_t meta_words, acc_stride;
   uint32_t stages;  // as many as fit, 0 when not even two do
-  bool hold;        // wide variant: sums staged in the ring stage of a tile's last row
+  bool hold;        // sums staged in the ring stage of a tile's last row (MayHold)
   size_t stage_bytes;
 };
 
@@ -2333,16 +2333,21 @@ PipeLayout MakePipeLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, uin
   off = align(off, 128);
   l.stage_bytes = runs * (1 + n_dir) * n_corr * 8;
   const size_t fit = off < dims.max_smem ? (dims.max_smem - off) / l.stage_bytes : 0;
-  // A deeper ring rather than a staging area where that leaves fewer than
-  // three stages: 256 stations, 16 directions, two stages and an area 211 us a
-  // pass, three without 178; 80 stations, 40 directions 92 and 93.
-  if (fit < 3 && !hold && warps == kWideWarps) {
-    const PipeLayout h = MakePipeLayout(dims, ng, warps, n_gbuf, stage_q, true);
-    if (h.stages > (fit < 2 ? 0 : fit)) return h;
-  }
   l.off_stages = uint32_t(off);
   l.stages = fit < 2 ? 0u : uint32_t(std::min<size_t>(fit, kPipeMaxStages));
   return l;
+}
+
+// The layout with one gain-table buffer: a deeper ring rather than a staging
+// area where that leaves fewer than three stages (256 stations, 16 directions,
+// two stages and an area 211 us a pass, three without 178; 80 stations, 40
+// directions 92 and 93; 512 stations, 5 directions, 32 rows a tile, two lanes per
+// run and an area 307, one lane without 277).
+PipeLayout DeepestLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, bool stage_q) {
+  const PipeLayout own = MakePipeLayout(dims, ng, warps, 1, stage_q);
+  if (own.stages >= 3 || !MayHold(int(warps), int(dims.n_corr), int(ng))) return own;
+  const PipeLayout held = MakePipeLayout(dims, ng, warps, 1, stage_q, true);
+  return held.stages > own.stages ? held : own;
 }
 
 // The pipe_kernel of a context: the fewest lanes per run that hold the
@@ -2367,7 +2372,7 @@ const KernelEntry* FindPipeKernel(const PipeDims& dims) {
       if (e.ncorr != int(dims.n_corr) || e.npol != int(dims.n_pol) || e.dmax != int(dpl) ||
           e.ng != int(ng))
         continue;
-      const uint32_t stages = MakePipeLayout(dims, ng, uint32_t(e.warps), 1, true).stages;
+      const uint32_t stages = DeepestLayout(dims, ng, uint32_t(e.warps), true).stages;
       if (stages <= best_stages || best_stages >= 3) continue;
       best = &e;
       best_stages = stages;
@@ -2915,8 +2920,8 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
       !std::getenv("DDSOLVE_NO_POWERS") && n_runs_all > 0 &&
       (ctx->tune_powers == 1 || (ctx->tune_powers < 0 && run_rows >= 16 * n_runs_all));
   if (use_powers && ctx->tune_powers < 0 && ctx->dmax <= kPipeDirs2) {
-    const PipeLayout l = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng,
-                                        uint32_t(ctx->pipe_entry->warps), 1, false);
+    const PipeLayout l =
+        DeepestLayout(DimsOf(ctx), ctx->pipe_ng, uint32_t(ctx->pipe_entry->warps), false);
     use_powers = !(l.hold && l.stages == 2);
   }
   // ---- fragments: rows balanced over the CTAs ----
@@ -3033,8 +3038,8 @@ int BuildPipePlan(ddsolve_ctx* ctx, std::vector<SlabDesc>& descs,
   uint32_t n_gbuf = ctx->tune_gbuf == 1 ? 1u : 2u;
   PipeLayout lay = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, n_gbuf, !use_powers);
   if (n_gbuf == 2 && lay.stages < (ctx->tune_gbuf == 2 ? 2u : 4u)) {
-    const PipeLayout one = MakePipeLayout(DimsOf(ctx), ctx->pipe_ng, warps, 1, !use_powers);
-    if (one.stages > lay.stages || (one.stages == lay.stages && lay.hold && !one.hold)) {
+    const PipeLayout one = DeepestLayout(DimsOf(ctx), ctx->pipe_ng, warps, !use_powers);
+    if (one.stages > lay.stages) {
       n_gbuf = 1;
       lay = one;
     }
@@ -4009,7 +4014,7 @@ int ddsolve_describe_layout(const ddsolve_dims* dims, ddsolve_layout* layout) {
     layout->pipelined = 1;
     layout->lanes_per_run = uint32_t(e->ng);
     layout->directions_per_lane = uint32_t(e->dmax);
-    layout->stages = MakePipeLayout(d, uint32_t(e->ng), uint32_t(e->warps), 1, true).stages;
+    layout->stages = DeepestLayout(d, uint32_t(e->ng), uint32_t(e->warps), true).stages;
   }
   return DDSOLVE_OK;
 }

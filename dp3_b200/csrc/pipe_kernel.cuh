@@ -93,7 +93,7 @@ struct PipeParams {
   uint32_t power_floats;  // floats per tile in `powers`
   // shared-memory layout (byte offsets)
   uint32_t off_acc, off_gtab, off_stg, off_q, off_meta, off_stages;
-  uint32_t hold;  // wide variant: no staging area (PipeLayout::hold)
+  uint32_t hold;  // no staging area (PipeLayout::hold)
   const FinList* fin_lists;    // [n_cb * n_sub]
   const uint32_t* fin_visits;
   uint32_t* cb_flag;     // channel block holds non-finite solutions
@@ -1202,16 +1202,25 @@ __device__ __forceinline__ void GatherTile(uint32_t meta_at, uint32_t gtab_at, u
 // (240 channels, 8 times) 6.27 -> 5.41 ms, over 12 blocks of 20 rows 2.13 -> 1.05.
 // SUMQ: the model powers are summed in the row loop (else precomputed).
 constexpr int kPairValues = 6;  // model values per lane up to which two rows fit its registers
-// Of a lane's directions, staged at a time: all, or in the wide variant what
-// the ring stage of a tile's last row holds too, where the sums are staged when
-// a ring of three stages leaves no room for an area of their own
-// (PipeLayout::hold): all of up to five directions (P and Q of two
-// polarizations: half of them), three of more (40 directions take 101 KB of
-// accumulators and gains). 512 stations, 16 directions, one polarization, 8
-// rows a tile: 214 us a pass staged in two rounds, 202 in one.
+// Of a lane's directions, staged at a time: all; in the wide variant of more
+// than kPipeDirs2 three (40 directions take 101 KB of accumulators and gains), and
+// of up to five with P and Q of two polarizations half of them. 512 stations, 16
+// directions, one polarization, 8 rows a tile: 214 us a pass in two rounds, 202
+// in one.
 __host__ __device__ constexpr int StageDirs(int warps, int dpl, int npol, bool sumq) {
   if (warps != kWideWarps) return 8;
   return dpl > int(kPipeDirs2) ? 3 : npol == 1 || !sumq ? dpl : (dpl + 1) / 2;
+}
+// Where a staging area of their own would leave a ring of fewer than three
+// stages, the sums are staged in the ring stage of the tile's last row
+// (PipeLayout::hold), as many directions at a time as it holds: on the variants
+// whose large arrays come to that, with two correlations.
+__host__ __device__ constexpr bool MayHold(int warps, int ncorr, int ng) {
+  return warps == kWideWarps || (ncorr == 2 && ng == 1);
+}
+__host__ __device__ constexpr int HeldDirs(int dpl, int npol, bool sumq) {
+  if (dpl > int(kPipeDirs2)) return 3;
+  return npol == 1 || !sumq || dpl == 1 ? dpl : dpl == 2 ? 1 : (dpl + 1) / 2;
 }
 __host__ __device__ constexpr uint32_t StagedBytes(uint32_t staged, uint32_t runs, uint32_t ncorr,
                                                    uint32_t npol) {  // of P
@@ -1231,7 +1240,8 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
   float* acc = reinterpret_cast<float*>(smem + p.off_acc);
   float2* gtab_buf = reinterpret_cast<float2*>(smem + p.off_gtab);
   constexpr int kStage = StageDirs(W, DPL, NPOL, SUMQ);
-  constexpr bool kMayHold = W == kWideWarps;
+  constexpr int kHeldStage = HeldDirs(DPL, NPOL, SUMQ);
+  constexpr bool kMayHold = MayHold(W, NCORR, NG);
   const bool hold = kMayHold && p.hold != 0;
   uint32_t* metas = reinterpret_cast<uint32_t*>(smem + p.off_meta);
   char* stages = reinterpret_cast<char*>(smem + p.off_stages);
@@ -1657,14 +1667,14 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
       uint32_t q_stage = 0;
       const uint32_t held = st == 0 ? S - 1 : st - 1;  // the last row's stage
       constexpr int kFewest = (DPL - 1) * NG + 1;  // directions of this variant
-      static_assert(!kMayHold || (kStage < DPL ? kStage * NG : kFewest) *
-                                         (NPOL == 1 ? 12 : SUMQ ? 12 * NCORR : 8 * NCORR) <=
-                                     (1 + kFewest) * int(E),
+      static_assert(!kMayHold || (kHeldStage < DPL ? kHeldStage * NG : kFewest) *
+                            (NPOL == 1 ? 12 : SUMQ ? 12 * NCORR : 8 * NCORR) <=
+                        (1 + kFewest) * int(E),
                     "the staged sums must fit in a held stage");
       const uint32_t stg_at =
           hold ? SmemAddr(stages + held * stage_bytes) : SmemAddr(smem) + p.off_stg;
       const uint32_t stg_q_at =
-          hold ? stg_at + StagedBytes(min(uint32_t(kStage * NG), n_dir), RUNS, NCORR, NPOL)
+          hold ? stg_at + StagedBytes(min(uint32_t(kHeldStage * NG), n_dir), RUNS, NCORR, NPOL)
                : SmemAddr(smem) + p.off_q;
       if (flags & kFragPower) {
         // the tile's precomputed model powers, in the stage after its rows
@@ -1680,54 +1690,65 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
       }
       float4* const stg = SharedPtr<float4>(stg_at);
       float2* const stg_q = SharedPtr<float2>(stg_q_at);
+      auto reduce = [&](auto at_a_time) {
+        constexpr int KS = decltype(at_a_time)::value;
 #pragma unroll
-      for (int k0 = 0; k0 < DPL; k0 += kStage) {
-        ConsumerBarrier<W>();  // the previous reduction is complete everywhere
-        if (active) {
+        for (int k0 = 0; k0 < DPL; k0 += KS) {
+          ConsumerBarrier<W>();  // the previous reduction is complete everywhere
+          if (active) {
 #pragma unroll
-          for (int k = k0; k < DPL && k < k0 + kStage; ++k) {
-            const uint32_t j = g + (k - k0) * NG;  // staged direction k0 * NG + j
-            if (k < DPL - 1 || last_mine) {
-              if constexpr (NPOL == 1) {
-                float3 v = make_float3(0.f, 0.f, 0.f);
+            for (int k = k0; k < DPL && k < k0 + KS; ++k) {
+              const uint32_t j = g + (k - k0) * NG;  // staged direction k0 * NG + j
+              if (k < DPL - 1 || last_mine) {
+                if constexpr (NPOL == 1) {
+                  float3 v = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
-                for (int c = 0; c < NCORR; ++c) {
-                  v.x += P[k][c].x;
-                  v.y += P[k][c].y;
-                  if constexpr (SUMQ) v.z += Q[k][c];
-                }
-                if (!SUMQ && q_src) {
-                  const float* q =
-                      SharedPtr<const float>(q_src) + ((g + k * NG) * RUNS + run) * NCORR;
+                  for (int c = 0; c < NCORR; ++c) {
+                    v.x += P[k][c].x;
+                    v.y += P[k][c].y;
+                    if constexpr (SUMQ) v.z += Q[k][c];
+                  }
+                  if (!SUMQ && q_src) {
+                    const float* q =
+                        SharedPtr<const float>(q_src) + ((g + k * NG) * RUNS + run) * NCORR;
 #pragma unroll
-                  for (int c = 0; c < NCORR; ++c) v.z += q[c];
-                }
-                reinterpret_cast<float2*>(stg)[j * RUNS + run] = make_float2(v.x, v.y);
-                reinterpret_cast<float*>(stg_q)[j * RUNS + run] = v.z;
-              } else {
-#pragma unroll
-                for (int h = 0; h < NCORR / 2; ++h)
-                  stg[(j * RUNS + run) * (NCORR / 2) + h] = make_float4(
-                      P[k][2 * h].x, P[k][2 * h].y, P[k][2 * h + 1].x, P[k][2 * h + 1].y);
-                if constexpr (SUMQ) {
+                    for (int c = 0; c < NCORR; ++c) v.z += q[c];
+                  }
+                  reinterpret_cast<float2*>(stg)[j * RUNS + run] = make_float2(v.x, v.y);
+                  reinterpret_cast<float*>(stg_q)[j * RUNS + run] = v.z;
+                } else {
 #pragma unroll
                   for (int h = 0; h < NCORR / 2; ++h)
-                    stg_q[(j * RUNS + run) * (NCORR / 2) + h] =
-                        make_float2(Q[k][2 * h], Q[k][2 * h + 1]);
+                    stg[(j * RUNS + run) * (NCORR / 2) + h] = make_float4(
+                        P[k][2 * h].x, P[k][2 * h].y, P[k][2 * h + 1].x, P[k][2 * h + 1].y);
+                  if constexpr (SUMQ) {
+#pragma unroll
+                    for (int h = 0; h < NCORR / 2; ++h)
+                      stg_q[(j * RUNS + run) * (NCORR / 2) + h] =
+                          make_float2(Q[k][2 * h], Q[k][2 * h + 1]);
+                  }
                 }
               }
             }
           }
+          ConsumerBarrier<W>();
+          const uint32_t d0 = k0 * NG;
+          const uint32_t n_staged = min(uint32_t(KS * NG), n_dir - d0);
+          const uint32_t q_from = NPOL == 1          ? stg_q_at
+                                  : q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4
+                                                   : q_src;
+          GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), stg_at, q_from,
+                                        SmemAddr(acc), ctid, n_dir, d0, n_staged, p.acc_stride,
+                                        p.gain_stride);
         }
-        ConsumerBarrier<W>();
-        const uint32_t d0 = k0 * NG;
-        const uint32_t n_staged = min(uint32_t(kStage * NG), n_dir - d0);
-        const uint32_t q_from = NPOL == 1          ? stg_q_at
-                                : q_src && !SUMQ ? q_src + d0 * NCORR * RUNS * 4
-                                                 : q_src;
-        GatherTile<W, NCORR, NPOL, RUNS>(SmemAddr(meta), SmemAddr(gtab), stg_at, q_from,
-                                      SmemAddr(acc), ctid, n_dir, d0, n_staged, p.acc_stride,
-                                      p.gain_stride);
+      };
+      if constexpr (kMayHold && kHeldStage < DPL && kHeldStage < kStage) {
+        if (hold)
+          reduce(std::integral_constant<int, kHeldStage>{});
+        else
+          reduce(std::integral_constant<int, kStage>{});
+      } else {
+        reduce(std::integral_constant<int, kStage>{});
       }
       // (this thread's sums in the held stage, before a copy overwrites them)
       if (hold) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

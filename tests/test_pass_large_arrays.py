@@ -1,6 +1,6 @@
-"""The pipelined pass of 13 to 48 directions at the sizes where its layout
-changes: the wide variant for up to 20 directions, and tiles whose sums are
-staged in the ring stage of their last row, up to the largest array that fits.
+"""The pipelined pass at the sizes where its layout changes: the wide variant
+for 13 to 20 directions, and tiles whose sums are staged in the ring stage of
+their last row, up to the largest array that fits.
 
 Tolerance: as for every pass, 1e-4 of the FP64 oracle.
 """
@@ -17,7 +17,7 @@ RTOL = 1e-4
 @pytest.mark.parametrize("powers", [0, 1])
 @pytest.mark.parametrize("npol,n_dir,n_st", [
     (2, 20, 140), (2, 16, 256), (2, 16, 295), (2, 13, 374), (2, 20, 229), (2, 21, 219),
-    (2, 40, 95), (2, 48, 72), (1, 16, 512), (1, 16, 576), (1, 20, 468), (1, 36, 223)])
+    (2, 5, 400), (2, 5, 512), (2, 4, 600), (1, 5, 900), (2, 40, 95), (2, 48, 72), (1, 16, 512), (1, 16, 576), (1, 20, 468), (1, 36, 223)])
 def test_pass_and_solve(built, npol, n_dir, n_st, powers):
     from dp3_b200 import ddsolve
     n_cb, n_it = 2, 3
