@@ -2345,7 +2345,7 @@ PipeLayout MakePipeLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, uin
 // run and an area 307, one lane without 277).
 PipeLayout DeepestLayout(const PipeDims& dims, uint32_t ng, uint32_t warps, bool stage_q) {
   const PipeLayout own = MakePipeLayout(dims, ng, warps, 1, stage_q);
-  if (own.stages >= 3 || !MayHold(int(warps), int(dims.n_corr), int(ng))) return own;
+  if (own.stages >= 3 || !MayHold(int(warps), int(dims.n_corr), int(dims.n_pol), int(ng))) return own;
   const PipeLayout held = MakePipeLayout(dims, ng, warps, 1, stage_q, true);
   return held.stages > own.stages ? held : own;
 }
@@ -3817,7 +3817,7 @@ int LaunchFullJones(ddsolve_ctx* ctx, bool host_mode, bool use_handle, bool with
 // Passes of one launch of pipe_kernel (see kLaunchBytes).
 uint32_t PassesPerLaunch(const ddsolve_ctx* ctx) {
   const double n = kLaunchBytes / std::max(ctx->pass_bytes, 1.0);
-  return n < 1.0 ? 1u : uint32_t(std::min<double>(n, kItersPerLaunch));
+  return uint32_t(std::min<double>(std::max<double>(n, kItersAtLeast), kItersPerLaunch));
 }
 
 // `n_passes` (pipe_kernel, without constraints): passes of the one launch --

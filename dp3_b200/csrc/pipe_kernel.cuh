@@ -56,8 +56,9 @@ constexpr uint32_t kVerdictNear = 2u;  // it may end with the next one
 // two. 62 stations, 10 directions, 50 passes of 637 MB: a launch more adds 16 us
 // to a solve of 5.36 ms; with the next interval's upload and predict on a second
 // context an interval takes 8.7 to 9.5 ms with one launch a solve, 7.9 to 8.1
-// with 9 GB, 7.7 with 6 or 4 GB.
-constexpr uint32_t kItersPerLaunch = 64;
+// with 9 GB, 7.7 with 6 or 4 GB. At least ten passes, so that the
+// launches cost no more than half a percent of a large array's solve.
+constexpr uint32_t kItersPerLaunch = 64, kItersAtLeast = 10;
 constexpr double kLaunchBytes = 9e9;
 
 // The partial slots of one (channel block, sub-solution) in the finalisation:
@@ -1214,9 +1215,11 @@ __host__ __device__ constexpr int StageDirs(int warps, int dpl, int npol, bool s
 // Where a staging area of their own would leave a ring of fewer than three
 // stages, the sums are staged in the ring stage of the tile's last row
 // (PipeLayout::hold), as many directions at a time as it holds: on the variants
-// whose large arrays come to that, with two correlations.
-__host__ __device__ constexpr bool MayHold(int warps, int ncorr, int ng) {
-  return warps == kWideWarps || (ncorr == 2 && ng == 1);
+// whose large arrays come to that and gain by it, all with two correlations (one
+// polarization and one lane per run: 900 stations, 5 directions 162 us a pass,
+// 159 on two lanes).
+__host__ __device__ constexpr bool MayHold(int warps, int ncorr, int npol, int ng) {
+  return warps == kWideWarps || (ncorr == 2 && npol == 2 && ng == 1);
 }
 __host__ __device__ constexpr int HeldDirs(int dpl, int npol, bool sumq) {
   if (dpl > int(kPipeDirs2)) return 3;
@@ -1241,7 +1244,7 @@ __global__ void __launch_bounds__(W * 32 + 32, 1) pipe_kernel(const PipeParams p
   float2* gtab_buf = reinterpret_cast<float2*>(smem + p.off_gtab);
   constexpr int kStage = StageDirs(W, DPL, NPOL, SUMQ);
   constexpr int kHeldStage = HeldDirs(DPL, NPOL, SUMQ);
-  constexpr bool kMayHold = MayHold(W, NCORR, NG);
+  constexpr bool kMayHold = MayHold(W, NCORR, NPOL, NG);
   const bool hold = kMayHold && p.hold != 0;
   uint32_t* metas = reinterpret_cast<uint32_t*>(smem + p.off_meta);
   char* stages = reinterpret_cast<char*>(smem + p.off_stages);

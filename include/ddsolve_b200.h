@@ -513,7 +513,7 @@ DDSOLVE_API int ddsolve_check_wait_limit(ddsolve_ctx* ctx, uint32_t wait_ms);
 
 /* Number of kernel launches issued by the last ddsolve_solve call (an
  * unconstrained solve on the pipelined path runs up to 64 iterations in one,
- * fewer where their visibilities exceed 9 GB). */
+ * fewer, but ten, where their visibilities exceed 9 GB). */
 DDSOLVE_API uint64_t ddsolve_last_launch_count(const ddsolve_ctx* ctx);
 
 #ifdef __cplusplus
